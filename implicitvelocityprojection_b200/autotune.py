@@ -148,22 +148,22 @@ def tune(scenes: Sequence, device: str = "cuda", base_options=None, warmup: int 
     rfs = ROW_FORMATS if base.row_format in (0, 1, 2) else (base.row_format,)
     for g, t, pers, rf in candidates(per_phase, rfs):
         ms = _time_candidate(scenes, g, t, pers, rf, device, warmup, steps, base)
-        trials.append(Trial(g, t, pers, rf, ms))
+        trials.append(Trial(g, t, pers, rf, round(ms, 4)))  # as reported: ties go to the first in the table
     best = min(trials, key=lambda tr: tr.ms_per_step)
     build_ms = None
     if base.build_kernel == 0:
         # both build kernels with the fastest shape, each build launch timed
         # inside steps (a caller that fixed the build kernel keeps it)
-        build_ms = {bk: _time_build(scenes, best.lanes_per_particle, best.particles_per_block, best.persistent,
-                                    best.row_format, bk, device, warmup, BUILD_REPS, base)
+        build_ms = {bk: round(_time_build(scenes, best.lanes_per_particle, best.particles_per_block, best.persistent,
+                                          best.row_format, bk, device, warmup, BUILD_REPS, base), 4)
                     for bk in BUILD_KERNELS}
     res = {"signature": key,
            "choice": {"lanes_per_particle": best.lanes_per_particle, "particles_per_block": best.particles_per_block,
                       "persistent": best.persistent, "row_format": best.row_format,
                       "build_kernel": min(build_ms, key=build_ms.get) if build_ms else base.build_kernel},
-           "table": [{"shape": tr.label(), "ms_per_step": round(tr.ms_per_step, 4)} for tr in trials],
+           "table": [{"shape": tr.label(), "ms_per_step": tr.ms_per_step} for tr in trials],
            "build_ms": None if build_ms is None else
-           {{1: "thread per particle", 2: "warp per cell"}[bk]: round(ms, 4) for bk, ms in build_ms.items()},
+           {{1: "thread per particle", 2: "warp per cell"}[bk]: ms for bk, ms in build_ms.items()},
            "tuning_s": round(time.perf_counter() - t0, 2), "steps_timed": steps}
     _CACHE[key] = res
     if cache_file:

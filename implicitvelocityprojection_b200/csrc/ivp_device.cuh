@@ -13,7 +13,8 @@
 //   * per-slot arrays: xm (float4 x,y,z,m), rest density, density, k, c, and
 //     the solver vectors as float4 (16-byte gathers);
 //   * neighbour rows, one per dynamic particle, `stride` entries of float4
-//     {J_ij, neighbour slot}: J_ij = m_j grad W_ij, the per-pair vector the
+//     {J_ij, neighbour slot}, interleaved so that a warp reads its particles'
+//     rows in whole lines (row_entry): J_ij = m_j grad W_ij, the per-pair vector the
 //     reference forms from its cache (J_ij / val_ij in pressure_base.py:81
 //     and ip.py:54; spiky gradient of sph_kernel.py:52-61).  Every
 //     neighbour sum then streams its row and gathers only the neighbour's
@@ -34,6 +35,7 @@ namespace ivp {
 
 constexpr int kMaxHistDefault = 128;
 constexpr int SOLVER_IP = 0, SOLVER_PRJ = 1;
+constexpr int BAR_VISC = 0, BAR_ST = 1, BAR_IP = 2, BAR_PRJ = 3, kBarrierWords = 4;
 
 struct SceneParams {
     int p_begin, p_end;        // particle range in the bound arrays
@@ -149,10 +151,6 @@ struct Dev {
     int n_scenes;
     SceneCtl* ctl;
     const int4* tiles;       // (scene, slot begin, slot end, row begin)
-    const int4* segs;        // neighbour-build cell segments (scene, cy, cz, x_lo)
-    int n_segs;
-    int* live_segs;          // segments holding dynamic particles in the current build (any order)
-    int* seg_ctr;            // [0] live segment count
     int n_tiles;
     const int* pscene;       // scene of each particle
     // sort
@@ -209,6 +207,7 @@ struct Dev {
     float4* rip;
     float4* pip;
     float* jp;
+    float* jd;               // J d of the last pack or PRJ tail (own slot; only with a divergence output)
     // viscosity and surface-tension CG, per slot (own): the direction p and
     // the neighbour sum of the last phase A (L(p) or S(p), carried by the
     // recurrence L(p_k) = L(z_k) + beta L(p_(k-1)))
@@ -236,7 +235,8 @@ struct Dev {
     int row_fmt;
     int row_stream;          // 1: the rows exceed L2 (row loads hint L2 evict-first)
     int* nbr_cnt;
-    int stride;
+    int stride;              // entries per row, a multiple of 16 (a pair of each of 8 lanes)
+    int lg;                  // log2 of the lanes per particle: the interleaving of the rows (row_entry)
     // reductions
     double* partial;
     int* scene_counter;
@@ -260,7 +260,9 @@ struct Dev {
     int visc_enabled;
     int force;               // implicit non-pressure solve of this launch: 0 viscosity, 1 surface tension
     int bar_all_reduce;      // persistent solve: every CTA reduces the (few) partials itself
-    // persistent solve: grid-barrier words and the phase budget
+    // persistent solve: grid-barrier words and the phase budget.  Every kind of
+    // solve has its own arrival counter (a launch's copy of Dev points to its
+    // kind's), zero between calls
     unsigned* bar_count;
     unsigned* bar_gen;
     long long phase_limit;
@@ -344,23 +346,40 @@ __device__ __forceinline__ float group_sum(float v) {
 }
 
 constexpr int ROW_FULL = 0, ROW_COMPACT = 1, ROW_BF16 = 2;
+// How a kernel reads the rows: full rows that stay in L2, full rows that
+// stream from DRAM (Dev::row_stream), or whatever Dev::row_fmt says.
+constexpr int READ_FULL = 0, READ_STREAM = 1, READ_ANY = 2;
+
 
 __device__ __forceinline__ float bf16_lo(unsigned w) { return __uint_as_float(w << 16); }
 __device__ __forceinline__ float bf16_hi(unsigned w) { return __uint_as_float(w & 0xffff0000u); }
 __device__ __forceinline__ unsigned short bf16_bits(float f) { return __bfloat16_as_ushort(__float2bfloat16_rn(f)); }
 
-// Entry k of a neighbour row in any layout: full rows hold {J_ij, j},
+// Entry u of a lane, from its first one on: two and two side by side.
+__host__ __device__ constexpr int lane_entry(int u) { return (u >> 1) * 64 + (u & 1); }
+
+// Index of entry k of a neighbour row.  The rows of the 32 / G particles that
+// one warp works on (a slice) are interleaved: lane r G + l holds entries 2 l,
+// 2 l + 1, then 2 l + 2 G, ... of the slice's particle r, in pairs.  One 256-bit
+// load per lane reads a pair of every lane, 1 KB side by side.  Row-major rows
+// instead made a warp touch 32 / G separate places per load.
+__device__ __forceinline__ size_t row_entry(const Dev& D, int row, int k) {
+    const int r = row & ((32 >> D.lg) - 1), lane = (r << D.lg) + ((k >> 1) & ((1 << D.lg) - 1));
+    return (size_t)(row - r) * D.stride + ((k >> (1 + D.lg)) << 6) + 2 * lane + (k & 1);
+}
+
+// Entry k of a neighbour row in any format: full rows hold {J_ij, j},
 // compact rows {j, w_ij} with J_ij = w_ij (x_i - x_j), bf16 rows j and J_ij
 // rounded to bf16.
 __device__ __forceinline__ int row_j(const Dev& D, int row, int k) {
-    const size_t e = (size_t)row * D.stride + k;
+    const size_t e = row_entry(D, row, k);
     if (D.row_fmt == ROW_FULL) return __float_as_int(D.nbr[e].w);
     if (D.row_fmt == ROW_COMPACT) return __float_as_int(reinterpret_cast<const float2*>(D.nbr)[e].x);
     return reinterpret_cast<const int*>(D.nbr)[e];
 }
 
 __device__ __forceinline__ float3 row_J(const Dev& D, int row, int k, float3 xi, int* j) {
-    const size_t e = (size_t)row * D.stride + k;
+    const size_t e = row_entry(D, row, k);
     if (D.row_fmt == ROW_FULL) {
         const float4 v = D.nbr[e];
         *j = __float_as_int(v.w);
@@ -376,6 +395,36 @@ __device__ __forceinline__ float3 row_J(const Dev& D, int row, int k, float3 xi,
     *j = __float_as_int(v.x);
     const float3 r = sub3(xi, f3(D.xm[*j]));
     return make_float3(__fmul_rn(v.y, r.x), __fmul_rn(v.y, r.y), __fmul_rn(v.y, r.z));
+}
+
+__device__ __forceinline__ void put_entry(const Dev& D, int row, int k, int j, float3 J, float w) {
+    const size_t e = row_entry(D, row, k);
+    if (D.row_fmt == ROW_FULL) {
+        D.nbr[e] = make_float4(J.x, J.y, J.z, __int_as_float(j));
+    } else if (D.row_fmt == ROW_COMPACT) {
+        reinterpret_cast<float2*>(D.nbr)[e] = make_float2(__int_as_float(j), w);
+    } else {
+        reinterpret_cast<int*>(D.nbr)[e] = j;
+        unsigned short* gb = D.nbr_g + 3 * e;
+        gb[0] = bf16_bits(J.x);
+        gb[1] = bf16_bits(J.y);
+        gb[2] = bf16_bits(J.z);
+    }
+}
+
+// Fills row entries cnt .. end - 1 with {self, J = 0}, which contribute exactly
+// 0 to every sum: `end` is slice_entries, so that the pair loops need no bounds
+// test.  Lanes `first`, `first + step`, ... of the particle
+// share the entries.
+__device__ __forceinline__ void put_pads(const Dev& D, int row, int cnt, int end, int self, int first, int step) {
+    for (int k = cnt + first; k < end; k += step) put_entry(D, row, k, self, make_float3(0.f, 0.f, 0.f), 0.0f);
+}
+
+// Entries of a row of a slice whose largest row count is cnt_max: whole pairs of
+// every lane.
+__device__ __forceinline__ int slice_entries(const Dev& D, int cnt_max) {
+    const int g = 2 << D.lg;
+    return (cnt_max + g - 1) & ~(g - 1);
 }
 
 // One 32-byte CG record (two float4, 32-byte aligned) in a single 256-bit
@@ -399,7 +448,7 @@ __device__ __forceinline__ float4 ld_vec(const float4* p) {
     return a;
 }
 
-// Two consecutive neighbour-list entries (32-byte aligned, read-only for the
+// Two consecutive neighbour-row entries (32-byte aligned, read-only for the
 // launch) in one 256-bit load through the non-coherent path.  A row is read
 // once per pass, so it does not allocate in L1, which keeps L1 for the
 // neighbour records that the particles of a tile share.

@@ -62,7 +62,7 @@ struct ivp_engine {
     ivp_options opt{};
     Dev D{};
     int G = 4, BLOCK = 128, T = 32;
-    int n_total = 0, n_dyn_total = 0, n_keys = 0, n_tiles = 0, scan_blocks = 0, n_segs = 0;
+    int n_total = 0, n_dyn_total = 0, n_keys = 0, n_tiles = 0, scan_blocks = 0;
     int fix_scan_blocks = 0;
     int* h_ovf = nullptr;        // pinned: truncated-list count read back by host-driven builds
     int* h_fix_scene = nullptr;  // pinned, n_scenes: corrections per scene
@@ -238,47 +238,52 @@ struct Launcher {
     }
 };
 
-template <int G, int BLOCK>
-struct Kern {
-    static DevKernel pack() { return k_pack<G, BLOCK>; }
-    static DevKernel rhs() { return k_rhs<G, BLOCK>; }
-    static DevKernel cg_a() { return k_cg_a<G, BLOCK>; }
-    static DevKernel cg_b() { return k_cg_b<G, BLOCK>; }
-    static DevKernel dens() { return k_density<G, BLOCK>; }
-    static DevKernel aii() { return k_aii<G, BLOCK>; }
-    static DevKernel div() { return k_divergence<G, BLOCK>; }
+struct KernelSet {
+    DevKernel pack, rhs, cg_a, cg_b, dens, aii, div, v_setup, v_a, v_b, v_end, st_div, pj_head, pj_tail;
+    DevKernel persist, v_persist, st_persist, prj_persist;  // for the engine's row format
+    size_t persist_smem;
 };
 
-struct KernelSet {
-    DevKernel pack, rhs, cg_a, cg_b, dens, aii, div, persist, v_setup, v_a, v_b, v_end, v_persist, st_div,
-        st_persist, pj_head, pj_tail, prj_persist;
-};
+template <int G, int B, int F>
+void set_persistent(KernelSet& K, int n_scenes) {
+    K.persist = k_ip_persistent<G, B, F>;
+    K.v_persist = k_force_persistent<G, B, F, FORCE_VISC>;
+    K.st_persist = k_force_persistent<G, B, F, FORCE_ST>;
+    K.prj_persist = k_prj_persistent<G, B, F>;
+    K.persist_smem = Phaser<G, B, F>::shared_bytes(n_scenes);
+}
 
 template <int G, int B>
-KernelSet make_set() {
-    return {Kern<G, B>::pack(), Kern<G, B>::rhs(), Kern<G, B>::cg_a(), Kern<G, B>::cg_b(),
-            Kern<G, B>::dens(), Kern<G, B>::aii(), Kern<G, B>::div(), k_ip_persistent<G, B>,
-            k_visc_setup<G, B>, k_visc_a<G, B>, k_visc_b<G, B>, k_visc_end<G, B>,
-            k_force_persistent<G, B, FORCE_VISC>, k_st_div<G, B>, k_force_persistent<G, B, FORCE_ST>,
-            k_pj_head<G, B>, k_pj_tail<G, B>, k_prj_persistent<G, B>};
+KernelSet make_set(int read, int n_scenes) {
+    KernelSet K = {k_pack<G, B>, k_rhs<G, B>, k_cg_a<G, B>, k_cg_b<G, B>, k_density<G, B>, k_aii<G, B>,
+                   k_divergence<G, B>, k_visc_setup<G, B>, k_visc_a<G, B>, k_visc_b<G, B>, k_visc_end<G, B>,
+                   k_st_div<G, B>, k_pj_head<G, B>, k_pj_tail<G, B>};
+    if (read == READ_FULL) set_persistent<G, B, READ_FULL>(K, n_scenes);
+    else if (read == READ_STREAM) set_persistent<G, B, READ_STREAM>(K, n_scenes);
+    else set_persistent<G, B, READ_ANY>(K, n_scenes);
+    return K;
+}
+
+int row_read(const Dev& D) {
+    return D.row_fmt != ROW_FULL ? READ_ANY : D.row_stream ? READ_STREAM : READ_FULL;
 }
 
 // Instantiated launch shapes: G lanes per particle x {128, 256} threads.
-bool kernel_set(int G, int B, KernelSet* out) {
+bool kernel_set(int G, int B, int read, int n_scenes, KernelSet* out) {
     if (B == 128) {
         switch (G) {
-            case 1: *out = make_set<1, 128>(); return true;
-            case 2: *out = make_set<2, 128>(); return true;
-            case 4: *out = make_set<4, 128>(); return true;
-            case 8: *out = make_set<8, 128>(); return true;
+            case 1: *out = make_set<1, 128>(read, n_scenes); return true;
+            case 2: *out = make_set<2, 128>(read, n_scenes); return true;
+            case 4: *out = make_set<4, 128>(read, n_scenes); return true;
+            case 8: *out = make_set<8, 128>(read, n_scenes); return true;
             default: return false;
         }
     }
     if (B == 256) {
         switch (G) {
-            case 2: *out = make_set<2, 256>(); return true;
-            case 4: *out = make_set<4, 256>(); return true;
-            case 8: *out = make_set<8, 256>(); return true;
+            case 2: *out = make_set<2, 256>(read, n_scenes); return true;
+            case 4: *out = make_set<4, 256>(read, n_scenes); return true;
+            case 8: *out = make_set<8, 256>(read, n_scenes); return true;
             default: return false;
         }
     }
@@ -342,13 +347,7 @@ int emit_build_impl(ivp_engine* e, Launcher& L, bool with_advect) {
             }
         }
     } else {
-        CKS(L.memset0(D.overflow, sizeof(int) * (size_t)e->n_scenes));
-        CKS(L.memset0(D.pairs, sizeof(unsigned long long) * (size_t)e->n_scenes));
-        CKS(L.memset0(D.seg_ctr, sizeof(int)));
-        CKS(L.memset0(D.ovf_ctr, 4 * sizeof(int)));
-        CKS(L.memset0(D.fix_fail, sizeof(int) * (size_t)e->n_scenes));
-        CKS(L.memset0(D.fix_scene, sizeof(int) * (size_t)e->n_scenes));
-        CKS(L.dev(IVP_K_KEYS, k_keys, blocks_for(e->n_total, ELEM_BLOCK), ELEM_BLOCK, D));
+        CKS(L.dev(IVP_K_KEYS, k_keys, blocks_for(std::max(e->n_total, e->n_scenes), ELEM_BLOCK), ELEM_BLOCK, D));
     }
     {
         int* in = D.cell_count;
@@ -361,9 +360,9 @@ int emit_build_impl(ivp_engine* e, Launcher& L, bool with_advect) {
         void* a2[] = {&out, &bs, &n, &nb};
         CKS(L.kernel(IVP_K_SCAN_ADD, (const void*)k_scan_add, dim3(e->scan_blocks), dim3(SCAN_BLOCK), a2));
     }
-    CKS(L.dev(IVP_K_PLACE, k_place, blocks_for(std::max(e->n_total, e->n_segs), ELEM_BLOCK), ELEM_BLOCK, D));
+    CKS(L.dev(IVP_K_PLACE, k_place, blocks_for(e->n_total, ELEM_BLOCK), ELEM_BLOCK, D));
     CKS(L.dev(IVP_K_ORDER, k_order, blocks_for(e->n_total, ELEM_BLOCK), ELEM_BLOCK, D));
-    if (e->n_segs > 0 && e->n_tiles > 0) {
+    if (e->n_tiles > 0) {
         Dev copy = D;
         cudaGraphConditionalHandle h_fix = 0;
         if (L.graph) {
@@ -371,15 +370,21 @@ int emit_build_impl(ivp_engine* e, Launcher& L, bool with_advect) {
             CK(cudaGraphConditionalHandleCreate(&h_fix, L.graph, 0, cudaGraphCondAssignDefault));
             copy.h_fix = (unsigned long long)h_fix;
         }
-        void* args[] = {&copy};
         if (e->opt.build_kernel == 2) {
-            // cell-tiled build: one CTA per segment holding dynamic particles
-            // (k_place listed them), one warp per cell
-            CKS(L.kernel(IVP_K_NBR_BUILD, (const void*)k_nbr_build<kBuildPP>, dim3(e->n_segs), dim3(256), args,
-                         sizeof(float4) * kStageCap));
+            // warps of eight slots, or of a slice of rows where that is more
+            const int sub = std::max(8, 32 / e->G);
+            const int warps = e->n_tiles * blocks_for(e->T, sub);
+            int T = e->T;
+            void* args[] = {&copy, &T};
+            CKS(L.kernel(IVP_K_NBR_BUILD,
+                         sub == 8    ? (const void*)k_nbr_build<8>
+                         : sub == 16 ? (const void*)k_nbr_build<16>
+                                     : (const void*)k_nbr_build<32>,
+                         dim3(blocks_for(warps, kBuildWarps)), dim3(32 * kBuildWarps), args));
         } else {
             // one thread per dynamic particle, one CTA per tile
             const int nt = std::max(e->T, 32);
+            void* args[] = {&copy};
             CKS(L.kernel(IVP_K_NBR_BUILD, (const void*)k_nbr_build_tpp, dim3(e->n_tiles), dim3(nt), args,
                          sizeof(unsigned short) * kTppHits * nt));
         }
@@ -418,7 +423,7 @@ int add_conditional(cudaGraph_t g, Launcher& L, cudaGraphConditionalHandle h, cu
 // (device-side control) or driven from the host with flag read-backs.
 int emit_solve_loop(ivp_engine* e, Launcher& L) {
     KernelSet K;
-    if (!kernel_set(e->G, e->BLOCK, &K)) return IVP_ERR_BAD_ARG;
+    if (!kernel_set(e->G, e->BLOCK, row_read(e->D), e->n_scenes, &K)) return IVP_ERR_BAD_ARG;
     const int nt = e->n_tiles, B = e->BLOCK;
     if (nt == 0) return IVP_OK;
     if (!L.graph) {
@@ -482,11 +487,11 @@ bool force_any(const ivp_engine* e, int force) { return force == FORCE_ST ? e->a
 int emit_prj(ivp_engine* e, Launcher& L) {
     if (e->n_tiles == 0 || !e->any_prj) return IVP_OK;
     KernelSet K;
-    if (!kernel_set(e->G, e->BLOCK, &K)) return IVP_ERR_BAD_ARG;
+    if (!kernel_set(e->G, e->BLOCK, row_read(e->D), e->n_scenes, &K)) return IVP_ERR_BAD_ARG;
     const int nt = e->n_tiles, B = e->BLOCK;
     if (e->persistent) {
-        CKS(L.memset0(e->D.bar_count, sizeof(unsigned)));
         Dev copy = e->D;
+        copy.bar_count += BAR_PRJ;
         void* args[] = {&copy};
         return L.kernel(IVP_K_PRJ, (const void*)K.prj_persist, dim3(e->coop_grid_prj), dim3(e->BLOCK), args,
                         e->coop_smem, true);
@@ -523,7 +528,7 @@ int emit_prj(ivp_engine* e, Launcher& L) {
 int emit_force(ivp_engine* e, Launcher& L, int force) {
     if (e->n_tiles == 0 || !force_any(e, force)) return IVP_OK;
     KernelSet K;
-    if (!kernel_set(e->G, e->BLOCK, &K)) return IVP_ERR_BAD_ARG;
+    if (!kernel_set(e->G, e->BLOCK, row_read(e->D), e->n_scenes, &K)) return IVP_ERR_BAD_ARG;
     const int nt = e->n_tiles, B = e->BLOCK;
     const int kid = force == FORCE_ST ? IVP_K_SURFACE_TENSION : IVP_K_VISC;
     Dev D0 = e->D;
@@ -562,9 +567,9 @@ int emit_solve(ivp_engine* e, Launcher& L, bool with_visc = false) {
     if (e->n_tiles == 0 || !e->any_ip) return IVP_OK;
     if (e->persistent) {
         KernelSet K;
-        kernel_set(e->G, e->BLOCK, &K);
-        CKS(L.memset0(e->D.bar_count, sizeof(unsigned)));
+        kernel_set(e->G, e->BLOCK, row_read(e->D), e->n_scenes, &K);
         Dev copy = e->D;
+        copy.bar_count += BAR_IP;
         copy.visc_enabled = with_visc ? 1 : 0;
         void* args[] = {&copy};
         return L.kernel(IVP_K_PERSISTENT, (const void*)K.persist, dim3(e->coop_grid), dim3(e->BLOCK), args,
@@ -575,7 +580,7 @@ int emit_solve(ivp_engine* e, Launcher& L, bool with_visc = false) {
     CKS(L.dev(IVP_K_SOLVE_END, k_solve_end, e->n_tiles, e->T, e->D));
     if (e->want_divergence && e->D.div_out) {
         KernelSet K;
-        kernel_set(e->G, e->BLOCK, &K);
+        kernel_set(e->G, e->BLOCK, row_read(e->D), e->n_scenes, &K);
         CKS(L.dev(IVP_K_DIVERGENCE, K.div, e->n_tiles, e->BLOCK, e->D));
     }
     return IVP_OK;
@@ -588,9 +593,9 @@ int emit_advect(ivp_engine* e, Launcher& L) {
 int emit_force_persistent(ivp_engine* e, Launcher& L, int force, bool fold_gravity = false) {
     if (e->n_tiles == 0 || !force_any(e, force)) return IVP_OK;
     KernelSet K;
-    kernel_set(e->G, e->BLOCK, &K);
-    CKS(L.memset0(e->D.bar_count, sizeof(unsigned)));
+    kernel_set(e->G, e->BLOCK, row_read(e->D), e->n_scenes, &K);
     Dev copy = e->D;
+    copy.bar_count += force == FORCE_ST ? BAR_ST : BAR_VISC;
     copy.force = force;
     copy.fold_gravity = fold_gravity && force == FORCE_VISC ? 1 : 0;
     if (force == FORCE_ST)
@@ -744,7 +749,7 @@ int validate(const ivp_scene_desc* sc, int n, const ivp_options* o) {
         return IVP_ERR_BAD_ARG;
     {
         KernelSet K;
-        if (o->particles_per_block <= 0 || !kernel_set(o->lanes_per_particle, o->particles_per_block * o->lanes_per_particle, &K))
+        if (o->particles_per_block <= 0 || !kernel_set(o->lanes_per_particle, o->particles_per_block * o->lanes_per_particle, READ_FULL, n, &K))
             return IVP_ERR_BAD_ARG;
     }
     if (o->list_stride <= 0 || (o->list_stride & 1) || o->max_hist <= 0) return IVP_ERR_BAD_ARG;
@@ -774,8 +779,9 @@ bool scene_st(const ivp_scene_desc& d) {
 struct Plan {
     std::vector<SceneParams> hp;
     std::vector<int4> tiles;
-    std::vector<int4> segs;
     int n_total = 0, n_dyn = 0, n_keys = 0, scan_blocks = 0;
+    int n_rows = 0;        // neighbour rows: each scene's dynamic particles, rounded up to whole tiles
+    int stride = 0;        // entries per row: list_stride rounded up to 16, a pair of each of 8 lanes
     int row_fmt = 0;       // ROW_FULL (16 B entries), ROW_COMPACT ({j, w}, 8 B), ROW_BF16 (4 B id + 6 B)
     bool any_st = false;   // some scene runs the implicit surface tension
     int drop_cap = 0;      // dropped-pair records of the overflow fix-up
@@ -808,14 +814,7 @@ void plan(const ivp_scene_desc* sc, int n, const ivp_options* o, Plan& P) {
         q.h = h;
         q.cell_inv = 1.0f / h;
         q.inv_h = 1.0f / h;
-        {
-            // largest float d2 with sqrtf(d2) < h (IEEE sqrt is monotone and
-            // correctly rounded on host and device alike)
-            float t = h * h;
-            while (std::sqrt(t) >= h) t = std::nextafter(t, 0.0f);
-            while (std::sqrt(std::nextafter(t, INFINITY)) < h) t = std::nextafter(t, INFINITY);
-            q.r2_max = t;
-        }
+        q.r2_max = strict_r2_max(h);
         long ncell = 1;
         for (int a = 0; a < 3; ++a) {
             // neighbour_search.py:105-107
@@ -856,16 +855,15 @@ void plan(const ivp_scene_desc* sc, int n, const ivp_options* o, Plan& P) {
             P.tiles.push_back(make_int4(s, s_begin + b, s_begin + e, row_base + b));
         }
         q.tile_end = (int)P.tiles.size();
-        if (d.n_dynamic > 0)
-            for (int cz = 0; cz < q.dims[2]; ++cz)
-                for (int cy = 0; cy < q.dims[1]; ++cy)
-                    for (int x = 0; x < q.dims[0]; x += kSegW) P.segs.push_back(make_int4(s, cy, cz, x));
         s_begin += d.n_particles;
-        row_base += d.n_dynamic;
+        // whole tiles: the rows of one warp's particles are interleaved
+        row_base += (d.n_dynamic + T - 1) / T * T;
+        P.n_dyn += d.n_dynamic;
         key_base += 2 * (int)ncell;
     }
     P.n_total = s_begin;
-    P.n_dyn = row_base;
+    P.n_rows = row_base;
+    P.stride = (o->list_stride + 15) & ~15;
     // compact rows halve the list memory; they cost one more gather per
     // pair, which outweighs the halved list stream on B200, so the default
     // is full rows.  bf16 rows (10 B per entry) are the reduced-precision
@@ -906,8 +904,8 @@ void plan(const ivp_scene_desc* sc, int n, const ivp_options* o, Plan& P) {
     P.off[i++] = L.add(sizeof(float) * N);                  // 25 s
     P.off[i++] = L.add(sizeof(float) * N);                  // 26 fk
     const size_t entry_bytes = P.row_fmt == ROW_FULL ? sizeof(float4) : P.row_fmt == ROW_COMPACT ? sizeof(float2) : sizeof(int);
-    P.off[i++] = L.add(entry_bytes * (size_t)P.n_dyn * (size_t)o->list_stride);  // 27 nbr (ids for bf16 rows)
-    P.off[i++] = L.add(sizeof(int) * std::max<size_t>((size_t)P.n_dyn, 1));       // 28 nbr_cnt
+    P.off[i++] = L.add(entry_bytes * (size_t)P.n_rows * (size_t)P.stride);  // 27 nbr (ids for bf16 rows)
+    P.off[i++] = L.add(sizeof(int) * std::max<size_t>((size_t)P.n_rows, 1));      // 28 nbr_cnt
     P.off[i++] = L.add(4 * sizeof(double) * NT);            // 29 partial (two per tile, two phase buffers)
     P.off[i++] = L.add(sizeof(int) * S);                    // 30 scene_counter
     P.off[i++] = L.add(sizeof(int));                        // 31 launch_counter
@@ -915,7 +913,7 @@ void plan(const ivp_scene_desc* sc, int n, const ivp_options* o, Plan& P) {
     P.off[i++] = L.add(sizeof(double) * S * (size_t)o->max_hist);  // 33 err_hist
     P.off[i++] = L.add(sizeof(int) * S * (size_t)o->max_hist);     // 34 pcg_hist
     P.off[i++] = L.add(sizeof(unsigned long long) * S);            // 35 pairs
-    P.off[i++] = L.add(2 * sizeof(unsigned));                        // 36 barrier words
+    P.off[i++] = L.add((kBarrierWords + 1) * sizeof(unsigned));      // 36 barrier words (counters, generation)
     P.off[i++] = L.add(sizeof(float) * N);                           // 37 inv_m
     P.off[i++] = L.add(sizeof(float) * N);                           // 38 q
     P.off[i++] = L.add(sizeof(float) * N);                           // 39 z
@@ -923,35 +921,33 @@ void plan(const ivp_scene_desc* sc, int n, const ivp_options* o, Plan& P) {
     P.off[i++] = L.add(sizeof(float4) * N);                          // 41 vs
     P.off[i++] = L.add(sizeof(float4) * N);                          // 42 vap
     P.off[i++] = L.add(3 * sizeof(float4) * N);                      // 43 pinv
-    P.off[i++] = L.add(sizeof(int4) * std::max<size_t>(P.segs.size(), 1));  // 44 segs
-    P.off[i++] = L.add(P.any_st ? sizeof(float2) * (size_t)P.n_dyn * (size_t)o->list_stride : 0);  // 45 st_w
-    P.off[i++] = L.add(P.any_st ? 2 * sizeof(float4) * N : 0);       // 46 st_rec
-    P.off[i++] = L.add(P.any_st ? sizeof(float) * N : 0);            // 47 st_inv
-    P.off[i++] = L.add(P.row_fmt == ROW_BF16 ? 3 * sizeof(unsigned short) * (size_t)P.n_dyn * (size_t)o->list_stride
-                                             : 0);                   // 48 bf16 gradients
-    P.off[i++] = L.add(sizeof(int) * std::max<size_t>(P.segs.size(), 1));  // 49 live_segs
-    P.off[i++] = L.add(sizeof(int));                                         // 50 seg_ctr (live segment count)
-    P.off[i++] = L.add(sizeof(float4) * N);                                  // 51 e = d - sol
+    P.off[i++] = L.add(P.any_st ? sizeof(float2) * (size_t)P.n_rows * (size_t)P.stride : 0);  // 44 st_w
+    P.off[i++] = L.add(P.any_st ? 2 * sizeof(float4) * N : 0);       // 45 st_rec
+    P.off[i++] = L.add(P.any_st ? sizeof(float) * N : 0);            // 46 st_inv
+    P.off[i++] = L.add(P.row_fmt == ROW_BF16 ? 3 * sizeof(unsigned short) * (size_t)P.n_rows * (size_t)P.stride
+                                             : 0);                   // 47 bf16 gradients
+    P.off[i++] = L.add(sizeof(float4) * N);                                  // 48 e = d - sol
     // neighbour-cache overflow fix-up
     P.drop_cap = 2 * std::max(P.n_dyn, 1) + kDropFloor;
     P.fix_scan_blocks = std::max(1, (P.n_total + SCAN_TILE - 1) / SCAN_TILE);
-    P.off[i++] = L.add(sizeof(int) * std::max<size_t>((size_t)P.n_dyn, 1));   // 52 ovf_list
-    P.off[i++] = L.add(4 * sizeof(int));                                       // 53 ovf_ctr
-    P.off[i++] = L.add(sizeof(int2) * (size_t)P.drop_cap);                     // 54 drop
-    P.off[i++] = L.add(sizeof(float4) * (size_t)P.drop_cap);                   // 55 drop_w
-    P.off[i++] = L.add(sizeof(int) * N);                                       // 56 fix_cnt
-    P.off[i++] = L.add(sizeof(int) * (N + 1));                                 // 57 fix_off
-    P.off[i++] = L.add(sizeof(int) * (size_t)P.fix_scan_blocks);               // 58 fix_bsums
-    P.off[i++] = L.add(2 * sizeof(float4) * (size_t)P.drop_cap);               // 59 fix_w
-    P.off[i++] = L.add(sizeof(int) * S);                                       // 60 fix_fail
-    P.off[i++] = L.add(sizeof(int) * S);                                       // 61 fix_scene
-    P.off[i++] = L.add(sizeof(float4) * N);                                    // 62 rip
-    P.off[i++] = L.add(sizeof(float4) * N);                                    // 63 pip
-    P.off[i++] = L.add(sizeof(float) * N);                                     // 64 jp
-    P.off[i++] = L.add(sizeof(float4) * N);                                    // 65 vpp
-    P.off[i++] = L.add(sizeof(float4) * N);                                    // 66 vlp
-    P.off[i++] = L.add(P.any_st ? sizeof(float4) * N : 0);                     // 67 stz
-    P.off[i++] = L.add(StatStage(o->max_hist).total);                          // 68 stage
+    P.off[i++] = L.add(sizeof(int) * std::max<size_t>((size_t)P.n_dyn, 1));   // 49 ovf_list
+    P.off[i++] = L.add(4 * sizeof(int));                                       // 50 ovf_ctr
+    P.off[i++] = L.add(sizeof(int2) * (size_t)P.drop_cap);                     // 51 drop
+    P.off[i++] = L.add(sizeof(float4) * (size_t)P.drop_cap);                   // 52 drop_w
+    P.off[i++] = L.add(sizeof(int) * N);                                       // 53 fix_cnt
+    P.off[i++] = L.add(sizeof(int) * (N + 1));                                 // 54 fix_off
+    P.off[i++] = L.add(sizeof(int) * (size_t)P.fix_scan_blocks);               // 55 fix_bsums
+    P.off[i++] = L.add(2 * sizeof(float4) * (size_t)P.drop_cap);               // 56 fix_w
+    P.off[i++] = L.add(sizeof(int) * S);                                       // 57 fix_fail
+    P.off[i++] = L.add(sizeof(int) * S);                                       // 58 fix_scene
+    P.off[i++] = L.add(sizeof(float4) * N);                                    // 59 rip
+    P.off[i++] = L.add(sizeof(float4) * N);                                    // 60 pip
+    P.off[i++] = L.add(sizeof(float) * N);                                     // 61 jp
+    P.off[i++] = L.add(sizeof(float4) * N);                                    // 62 vpp
+    P.off[i++] = L.add(sizeof(float4) * N);                                    // 63 vlp
+    P.off[i++] = L.add(P.any_st ? sizeof(float4) * N : 0);                     // 64 stz
+    P.off[i++] = L.add(StatStage(o->max_hist).total);                          // 65 stage
+    P.off[i++] = L.add(sizeof(float) * N);                                     // 66 jd
 }
 
 cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
@@ -1140,7 +1136,7 @@ int ivp_engine_create(const ivp_scene_desc* scenes, int32_t n_scenes, const ivp_
     D.pcg_hist = reinterpret_cast<int*>(w + P.off[i++]);
     D.pairs = reinterpret_cast<unsigned long long*>(w + P.off[i++]);
     D.bar_count = reinterpret_cast<unsigned*>(w + P.off[i]);
-    D.bar_gen = reinterpret_cast<unsigned*>(w + P.off[i++]) + 1;
+    D.bar_gen = reinterpret_cast<unsigned*>(w + P.off[i++]) + kBarrierWords;
     D.inv_m = reinterpret_cast<float*>(w + P.off[i++]);
     D.q = reinterpret_cast<float*>(w + P.off[i++]);
     D.z = reinterpret_cast<float*>(w + P.off[i++]);
@@ -1148,13 +1144,10 @@ int ivp_engine_create(const ivp_scene_desc* scenes, int32_t n_scenes, const ivp_
     D.vs = reinterpret_cast<float4*>(w + P.off[i++]);
     D.vap = reinterpret_cast<float4*>(w + P.off[i++]);
     D.pinv = reinterpret_cast<float4*>(w + P.off[i++]);
-    D.segs = reinterpret_cast<int4*>(w + P.off[i++]);
     D.st_w = reinterpret_cast<float2*>(w + P.off[i++]);
     D.st_rec = reinterpret_cast<float4*>(w + P.off[i++]);
     D.st_inv = reinterpret_cast<float*>(w + P.off[i++]);
     D.nbr_g = reinterpret_cast<unsigned short*>(w + P.off[i++]);
-    D.live_segs = reinterpret_cast<int*>(w + P.off[i++]);
-    D.seg_ctr = reinterpret_cast<int*>(w + P.off[i++]);
     D.e = reinterpret_cast<float4*>(w + P.off[i++]);
     D.ovf_list = reinterpret_cast<int*>(w + P.off[i++]);
     D.ovf_ctr = reinterpret_cast<int*>(w + P.off[i++]);
@@ -1173,10 +1166,9 @@ int ivp_engine_create(const ivp_scene_desc* scenes, int32_t n_scenes, const ivp_
     D.vlp = reinterpret_cast<float4*>(w + P.off[i++]);
     D.stz = reinterpret_cast<float4*>(w + P.off[i++]);
     D.stage = reinterpret_cast<unsigned char*>(w + P.off[i++]);
+    D.jd = reinterpret_cast<float*>(w + P.off[i++]);
     D.drop_cap = P.drop_cap;
     e->fix_scan_blocks = P.fix_scan_blocks;
-    D.n_segs = (int)P.segs.size();
-    e->n_segs = D.n_segs;
     {
         long long lim = 64;
         for (int sc = 0; sc < n_scenes; ++sc)
@@ -1188,7 +1180,8 @@ int ivp_engine_create(const ivp_scene_desc* scenes, int32_t n_scenes, const ivp_
     D.n_scenes = n_scenes;
     D.n_tiles = e->n_tiles;
     D.n_keys = e->n_keys;
-    D.stride = opt->list_stride;
+    D.stride = P.stride;
+    D.lg = e->G == 8 ? 3 : e->G == 4 ? 2 : e->G == 2 ? 1 : 0;
     D.row_fmt = P.row_fmt;
     {
         // rows hold about half their stride in use; beyond the L2 they
@@ -1234,9 +1227,7 @@ int ivp_engine_create(const ivp_scene_desc* scenes, int32_t n_scenes, const ivp_
         (e->n_tiles && cudaMemcpyAsync((void*)D.tiles, P.tiles.data(), sizeof(int4) * e->n_tiles,
                                        cudaMemcpyHostToDevice, s) != cudaSuccess) ||
         (e->n_total && cudaMemcpyAsync((void*)D.pscene, pscene.data(), sizeof(int) * e->n_total,
-                                       cudaMemcpyHostToDevice, s) != cudaSuccess) ||
-        (e->n_segs && cudaMemcpyAsync((void*)D.segs, P.segs.data(), sizeof(int4) * e->n_segs,
-                                      cudaMemcpyHostToDevice, s) != cudaSuccess))
+                                       cudaMemcpyHostToDevice, s) != cudaSuccess))
         return fail(IVP_ERR_CUDA);
     // the host vectors go out of scope: make the copies complete first
     if (cudaStreamSynchronize(s) != cudaSuccess) return fail(IVP_ERR_CUDA);
@@ -1245,8 +1236,12 @@ int ivp_engine_create(const ivp_scene_desc* scenes, int32_t n_scenes, const ivp_
     if (opt->persistent && e->n_tiles > 0 && n_scenes <= 256) {
         int dev = 0, coop = 0, nsm = 0, per_sm = 0;
         KernelSet K;
-        kernel_set(e->G, e->BLOCK, &K);
-        e->coop_smem = (size_t)n_scenes * (2 * sizeof(double) + sizeof(SceneCtl) + 3 * sizeof(int)) + sizeof(int);
+        kernel_set(e->G, e->BLOCK, row_read(e->D), e->n_scenes, &K);
+        e->coop_smem = K.persist_smem;
+        for (DevKernel k : {K.persist, K.v_persist, K.st_persist, K.prj_persist})
+            if (cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e->coop_smem) !=
+                cudaSuccess)
+                return fail(IVP_ERR_CUDA);
         if (cudaGetDevice(&dev) == cudaSuccess &&
             cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) == cudaSuccess && coop &&
             cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
@@ -1362,7 +1357,7 @@ int ivp_compute_density(ivp_engine* e, void* stream) {
     if (!e) return IVP_ERR_BAD_ARG;
     if (!e->bound) return IVP_ERR_NOT_BOUND;
     KernelSet K;
-    kernel_set(e->G, e->BLOCK, &K);
+    kernel_set(e->G, e->BLOCK, row_read(e->D), e->n_scenes, &K);
     Launcher L;
     L.stream = as_stream(stream);
     return L.dev(IVP_K_PACK, K.dens, e->n_tiles, e->BLOCK, e->D);
@@ -1372,14 +1367,40 @@ int ivp_compute_aii(ivp_engine* e, void* stream) {
     if (!e) return IVP_ERR_BAD_ARG;
     if (!e->bound) return IVP_ERR_NOT_BOUND;
     KernelSet K;
-    kernel_set(e->G, e->BLOCK, &K);
+    kernel_set(e->G, e->BLOCK, row_read(e->D), e->n_scenes, &K);
     Launcher L;
     L.stream = as_stream(stream);
     CKS(L.dev(IVP_K_PACK, K.aii, e->n_tiles, e->BLOCK, e->D));
     return L.dev(IVP_K_STATIC_OUT, k_static_outputs, blocks_for(e->n_total, ELEM_BLOCK), ELEM_BLOCK, e->D);
 }
 
-int emit_ip_only(ivp_engine* e, Launcher& L) { return emit_solve(e, L, false); }
+// The barrier counters of a solve outside a step go back to zero (a step's
+// advection does it for its own solves).
+int emit_barrier_reset(ivp_engine* e, Launcher& L) {
+    return e->persistent ? L.memset0(e->D.bar_count, kBarrierWords * sizeof(unsigned)) : (int)IVP_OK;
+}
+
+int emit_ip_only(ivp_engine* e, Launcher& L) {
+    CKS(emit_solve(e, L, false));
+    return emit_barrier_reset(e, L);
+}
+
+int emit_prj_only(ivp_engine* e, Launcher& L) {
+    CKS(emit_prj(e, L));
+    return emit_barrier_reset(e, L);
+}
+
+// A non-pressure force on its own: the kernel of the step where the engine's
+// solves are persistent.  One launch per phase would come back to the host
+// after every CG iteration.
+int force_only(ivp_engine* e, int force, cudaStream_t s) {
+    if (!e->bound) return IVP_ERR_NOT_BOUND;
+    Launcher L;
+    L.stream = s;
+    if (!e->persistent) return emit_force(e, L, force);
+    CKS(emit_force_persistent(e, L, force));
+    return emit_barrier_reset(e, L);
+}
 
 int ivp_ip_solve(ivp_engine* e, void* stream) {
     if (!e) return IVP_ERR_BAD_ARG;
@@ -1388,23 +1409,17 @@ int ivp_ip_solve(ivp_engine* e, void* stream) {
 
 int ivp_prj_solve(ivp_engine* e, void* stream) {
     if (!e) return IVP_ERR_BAD_ARG;
-    return run(e, emit_prj, &e->graph_prj, &e->exec_prj, as_stream(stream));
+    return run(e, emit_prj_only, &e->graph_prj, &e->exec_prj, as_stream(stream));
 }
 
 int ivp_viscosity_solve(ivp_engine* e, void* stream) {
     if (!e) return IVP_ERR_BAD_ARG;
-    if (!e->bound) return IVP_ERR_NOT_BOUND;
-    Launcher L;
-    L.stream = as_stream(stream);
-    return emit_force(e, L, FORCE_VISC);
+    return force_only(e, FORCE_VISC, as_stream(stream));
 }
 
 int ivp_surface_tension_solve(ivp_engine* e, void* stream) {
     if (!e) return IVP_ERR_BAD_ARG;
-    if (!e->bound) return IVP_ERR_NOT_BOUND;
-    Launcher L;
-    L.stream = as_stream(stream);
-    return emit_force(e, L, FORCE_ST);
+    return force_only(e, FORCE_ST, as_stream(stream));
 }
 
 int ivp_apply_gravity(ivp_engine* e, void* stream) {

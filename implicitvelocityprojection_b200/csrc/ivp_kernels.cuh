@@ -3,8 +3,8 @@
 // Bandwidth-bound sparse neighbour sums on CUDA cores (no tensor cores: the
 // operator is a gather over ~30 neighbours per particle, ~1 flop/byte).
 // Every neighbour-sum kernel maps G lanes to one particle: lane l takes the
-// list entries 2l, 2l+1, then 2l+2G, ... (two entries per 256-bit row read)
-// and the group reduces with shuffles.  Reductions across particles are FP64
+// list entries 2l, 2l+1, then 2l+2G, ... (two entries per 256-bit row read, a
+// warp's reads side by side in memory) and the group reduces with shuffles.  Reductions across particles are FP64
 // per-tile partials, summed per scene in one fixed association.  With one
 // launch per phase, the last CTA of each scene sums them and runs the
 // scene's solver control (outer loop / CG decisions of ip.py:346-392 and
@@ -15,6 +15,7 @@
 #pragma once
 #include "ivp_device.cuh"
 #include "ivp_scan.cuh"
+#include "ivp_window.cuh"
 
 namespace ivp {
 
@@ -27,7 +28,6 @@ enum Kind {
     K_PJ_HEAD = 8, K_PJ_TAIL = 9
 };
 constexpr int FORCE_VISC = 0, FORCE_ST = 1;
-constexpr int MODE_IP = 0, MODE_FORCE = 1, MODE_PRJ = 3;
 
 constexpr int IVP_OK_ = 0, IVP_NOT_SPD_ = 1, IVP_NOT_CONVERGED_ = 2, IVP_NBR_OVERFLOW_ = 3, IVP_TIMEOUT_ = 6;
 
@@ -385,46 +385,37 @@ __device__ __forceinline__ void cell_key(const Dev& D, int p, int sc, float px, 
     D.rank[p] = atomicAdd(&D.cell_count[key], 1);
 }
 
+// The build's per-scene counters start from zero (read from the build kernel on).
+__device__ __forceinline__ void build_begin(const Dev& D, int p) {
+    if (p < D.n_scenes) {
+        D.overflow[p] = 0;
+        D.pairs[p] = 0ull;
+        D.fix_fail[p] = 0;
+        D.fix_scene[p] = 0;
+    }
+    if (p == 0) {
+        D.ovf_ctr[0] = 0;
+        D.ovf_ctr[1] = 0;
+    }
+}
+
 __global__ void k_keys(const Dev D) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    build_begin(D, p);
     if (p >= D.n_total) return;
     cell_key(D, p, D.pscene[p], D.x[3 * p], D.x[3 * p + 1], D.x[3 * p + 2]);
 }
 
-// Build segments: kSegW cells along x of one (y, z) cell row of a scene.
-constexpr int kSegW = 8;
-
-// Places every particle (thread p < n_total) and, once the cell starts are
-// known, appends the build segments that hold dynamic particles (thread
-// g < n_segs) to D.live_segs in any order, one atomic per warp; D.seg_ctr[0]
-// (zeroed before) ends as their count.  Most segments of a scene's grid are
-// empty (air above the fluid), so the build then runs only CTAs that work.
+// Places every particle at its cell's start plus its rank.
 __global__ void k_place(const Dev D) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p < D.n_total) {
-        const int key = D.key[p];
-        D.placed[D.cell_start[key] + D.rank[p]] = p;
-        // the scan has consumed the counts: every nonzero count belongs to
-        // some particle's key, so this leaves cell_count all zero for the
-        // next build (the workspace starts zeroed)
-        D.cell_count[key] = 0;
-    }
-    bool live = false;
-    if (p < D.n_segs) {
-        const int4 seg = D.segs[p];
-        const SceneParams& P = D.scenes[seg.x];
-        const int dimx = P.dims[0];
-        const int x_hi = min(seg.w + kSegW, dimx) - 1;
-        const int kd0 = P.key_base + (seg.z * P.dims[1] + seg.y) * dimx;
-        live = D.cell_start[kd0 + x_hi + 1] > D.cell_start[kd0 + seg.w];
-    }
-    const unsigned ball = __ballot_sync(0xffffffffu, live);
-    if (!ball) return;
-    const int lane = threadIdx.x & 31;
-    int base = 0;
-    if (lane == 0) base = atomicAdd(D.seg_ctr, __popc(ball));
-    base = __shfl_sync(0xffffffffu, base, 0);
-    if (live) D.live_segs[base + __popc(ball & ((1u << lane) - 1u))] = p;
+    if (p >= D.n_total) return;
+    const int key = D.key[p];
+    D.placed[D.cell_start[key] + D.rank[p]] = p;
+    // the scan has consumed the counts: every nonzero count belongs to
+    // some particle's key, so this leaves cell_count all zero for the
+    // next build (the workspace starts zeroed)
+    D.cell_count[key] = 0;
 }
 
 // Stable order inside each cell (by particle id), then gather the particle
@@ -457,277 +448,189 @@ __global__ void k_order(const Dev D) {
 // diagonal k = 1/(Aii + 1e-3) (pressure_base.py:49-87) and the constraint
 // c = rho - rho0 (pressure_base.py:169-184).
 //
-// Cell-tiled: one CTA per build segment that holds dynamic particles (CTA b
-// takes D.live_segs[b]; the grid covers every segment and the CTAs past the
-// live count return at once).  The CTA stages the candidates of the 9
-// neighbouring rows x {dynamic, static} -- 18 contiguous slot ranges covering
-// x_lo-1 .. x_hi+1 -- into shared memory with coalesced loads, together with
-// their cell starts.
+// One warp takes SUB consecutive dynamic slots (8, or a slice of rows where that
+// is more) and works in two passes.
 //
-// One warp per cell: the particles of a cell share their 27-cell candidate
-// window, so a warp takes up to PP particles of one cell and walks the window
-// once.  Each lane loads one candidate per round and tests it against all PP
-// particles; one warp ballot per particle orders that round's hits by
-// candidate, so each list keeps the sequential candidate order (rows dz, dy
-// ascending; dynamic cells before static cells; slots ascending) and the
-// first-cache_size truncation of the sequential scan.  The window is the
-// concatenation of the cell's 18 slot ranges, so rounds run over all 32
-// lanes across range ends; a lane finds its range by a binary search over
-// the range starts.  The dense pass (J, density, Aii) then runs 32/PP lanes
-// per particle.  Segments whose neighbourhood exceeds the staging capacity
-// read the candidates from global memory instead.
-constexpr int kStageCap = 2048;  // staged candidates per CTA (32 KB): with PP = 4, static + dynamic shared stay under 48 KB
-constexpr int kBuildPP = 4;      // particles per warp
+// Filter: the slots are sorted by cell, so the warp's particles are a few runs
+// of one cell each (or of a few thinly filled x-adjacent cells), and the
+// particles of a run share their window of cells.  The window is up to 18 slot
+// ranges (rows dz outer, dy inner; dynamic then static slots of the x-adjacent
+// cells), walked end to end in chunks of 32: a lane holds one candidate of the
+// chunk, all lanes test it against one particle of the run after another, and
+// one ballot per particle and chunk is the whole result.  The ballots are then
+// expanded into each particle's hit list (16 bits a hit: the range's ordinal and
+// the window position), in the sequential candidate order, so the first
+// cache_size kept are those of the sequential scan.
+//
+// Dense pass: eight lanes per particle walk its list and form the row entry,
+// density and Aii terms of every hit.
+//
+// For scenes of few particles per SM, which wait for one warp's chain of loads:
+// no staging and no CTA barrier before the first test.  Against one CTA per run
+// of eight cells with its candidates staged in shared memory: 8,192 particles
+// 33 us instead of 35, 31,007 particles 47 us instead of 52 (768: 27 and 25).
+constexpr int kBuildWarps = 2;  // warps per CTA
 
-template <int PP>
-__global__ void __launch_bounds__(256, 4) k_nbr_build(const Dev D) {
-    constexpr int NW = 8;          // warps per CTA
-    constexpr int NC = kSegW + 3;  // cell starts x_lo-1 .. x_hi+2
-    constexpr int HB = 64;         // hit buffer per particle (cap <= 64)
-    constexpr int LPP = 32 / PP;   // lanes per particle in the dense pass
-    static_assert(PP == 2 || PP == 4, "PP: 2 or 4 particles per warp (shared memory stays under 48 KB)");
-    extern __shared__ float4 stage[];
-    __shared__ int sh_cs[18][NC];
-    __shared__ int sh_off[18], sh_base[18];
-    __shared__ int sh_total, sh_pairs;
-    __shared__ int sh_vst[NW][32];  // per warp: window offset of each range, INT_MAX past the 18th
-    __shared__ int sh_rj[NW][18];   // first slot of each range in the window
-    __shared__ int sh_rs[NW][18];   // its stage index
-    __shared__ int hit_j[NW][PP][HB];
-    __shared__ short hit_s[NW][PP][HB];
-    if ((int)blockIdx.x >= D.seg_ctr[0]) return;  // past the live segments (block-uniform)
-    const int4 seg = D.segs[D.live_segs[blockIdx.x]];  // (scene, cy, cz, x_lo)
-    const int sc = seg.x, cy = seg.y, cz = seg.z, x_lo = seg.w;
-    const SceneParams& P = D.scenes[sc];
-    const int dimx = P.dims[0];
-    const int x_hi = min(x_lo + kSegW, dimx) - 1;
-    const int kd0 = P.key_base + (cz * P.dims[1] + cy) * dimx;
-    const int s0 = __ldg(D.cell_start + kd0 + x_lo), s1 = __ldg(D.cell_start + kd0 + x_hi + 1);
-    if (s0 == s1) return;  // no dynamic particle in this segment (block-uniform)
-    for (int e = threadIdx.x; e < 18 * NC; e += blockDim.x) {
-        const int q = e / NC, c = e % NC;
-        const int rr = q >> 1, pass = q & 1;
-        const int z = cz + rr / 3 - 1, y = cy + rr % 3 - 1;
-        const int x = x_lo - 1 + c;
-        int v = -1;
-        if (z >= 0 && z < P.dims[2] && y >= 0 && y < P.dims[1] && x >= 0 && x <= dimx)
-            v = __ldg(D.cell_start + P.key_base + (pass ? P.ncell : 0) + (z * P.dims[1] + y) * dimx + x);
-        sh_cs[q][c] = v;
-    }
-    if (threadIdx.x == 0) sh_pairs = 0;
-    __syncthreads();
-    const int ca = (x_lo > 0 ? x_lo - 1 : 0) - (x_lo - 1);
-    const int cb = (x_hi < dimx - 1 ? x_hi + 1 : dimx - 1) + 1 - (x_lo - 1);
-    if (threadIdx.x < 32) {
-        const int q = threadIdx.x;
-        int len = 0, b = 0;
-        if (q < 18) {
-            b = sh_cs[q][ca];
-            const int e = sh_cs[q][cb];
-            len = (b >= 0 && e >= b) ? e - b : 0;
-        }
-        int incl = len;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int t = __shfl_up_sync(0xffffffffu, incl, o);
-            if (q >= o) incl += t;
-        }
-        if (q < 18) {
-            sh_off[q] = incl - len;
-            sh_base[q] = b;
-        }
-        if (q == 31) sh_total = incl;
-    }
-    __syncthreads();
-    const bool staged = sh_total <= kStageCap;
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (staged) {
-        // one flat pass over the staged candidates (every thread's loads are
-        // independent); a binary search over the range offsets finds each
-        // candidate's range
-        const int total = sh_total;
-#pragma unroll 4
-        for (int k = threadIdx.x; k < total; k += blockDim.x) {
-            int q = 0;
-#pragma unroll
-            for (int st = 16; st > 0; st >>= 1)
-                if (q + st < 18 && sh_off[q + st] <= k) q += st;
-            stage[k] = __ldg(D.xm + sh_base[q] + (k - sh_off[q]));
-        }
-    }
-    __syncthreads();
+// All hits of one particle by the whole warp, straight from its window: for
+// windows that do not fit the filter pass.  Every lane returns the sums;
+// `entry(k, j, J, w)` is called by the lane of each kept hit.
+template <class Entry>
+__device__ __forceinline__ int scan_alone(const WindowGrid& W, int* list, int i, float4 xi, int3 cell, int cap,
+                                          int dyn_end, float h, float inv_h, float spk, float ck, HitSums& s,
+                                          Entry&& entry) {
+    const int lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1u;
-    const float h = P.h, inv_h = P.inv_h, r2max = P.r2_max, spk = P.spiky_k, ck = P.cubic_k;
-    const int dyn_end = P.s_dyn_end;
-    const int cap = min(min(P.cache, D.stride), HB);
-    const int ncell = x_hi - x_lo + 1;
-    // work items: (cell, run of up to PP of its dynamic particles), dealt to
-    // the warps round-robin; the segment's own cells are row q = 8
-    // (dz = dy = 0, dynamic), columns 1 .. ncell + 1
-    int nitems = 0;
-    for (int k = 0; k < ncell; ++k) nitems += (sh_cs[8][k + 2] - sh_cs[8][k + 1] + PP - 1) / PP;
-    int my_pairs = 0;
-    for (int it = w; it < nitems; it += NW) {
-        int k = 0, acc = 0, pb = 0, pe = 0;
-        for (; k < ncell; ++k) {
-            const int b = sh_cs[8][k + 1], e = sh_cs[8][k + 2];
-            const int nch = (e - b + PP - 1) / PP;
-            if (it < acc + nch) {
-                pb = b + (it - acc) * PP;
-                pe = min(pb + PP, e);
-                break;
+    int b, len;
+    window_range(W, cell.x, cell.x, cell.y, cell.z, lane, b, len);
+    int found = 0;
+    for (int q = 0; q < 18; ++q) {
+        const int jb = __shfl_sync(0xffffffffu, b, q), n = __shfl_sync(0xffffffffu, len, q);
+        for (int base = 0; base < n; base += 32) {
+            const int j = jb + base + lane;
+            bool in = false;
+            if (base + lane < n && j != i) {
+                const float4 xj = __ldg(W.xm + j);
+                in = norm2_rn(make_float3(xi.x - xj.x, xi.y - xj.y, xi.z - xj.z)) <= W.r2_max;
             }
-            acc += nch;
+            const unsigned ball = __ballot_sync(0xffffffffu, in);
+            const int at = found + __popc(ball & lt);
+            if (in && at < cap) list[at] = j;
+            found += __popc(ball);
         }
-        const int cx = x_lo + k;
-        const int c0 = (cx > 0 ? cx - 1 : 0) - (x_lo - 1);
-        const int c1 = (cx < dimx - 1 ? cx + 1 : dimx - 1) + 1 - (x_lo - 1);
-        // the cell's window: 18 ranges, concatenated in scan order
-        int L;
-        {
-            int len = 0, jb = 0, so = 0;
-            if (lane < 18) {
-                jb = sh_cs[lane][c0];
-                const int je = sh_cs[lane][c1];
-                len = (jb >= 0 && je > jb) ? je - jb : 0;
-                so = sh_off[lane] + (jb - sh_base[lane]);
-            }
-            int incl = len;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int t = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += t;
-            }
-            sh_vst[w][lane] = lane < 18 ? incl - len : INT_MAX;
-            if (lane < 18) {
-                sh_rj[w][lane] = jb;
-                sh_rs[w][lane] = so;
-            }
-            L = __shfl_sync(0xffffffffu, incl, 31);
-            __syncwarp();
-        }
-        const int np = pe - pb;
-        float3 xi[PP];
-        int cnt[PP];
-#pragma unroll
-        for (int p = 0; p < PP; ++p) {
-            xi[p] = f3(D.xm[pb + (p < np ? p : 0)]);
-            cnt[p] = 0;
-        }
-        // phase 1: filter
-        for (int base = 0; base < L; base += 32) {
-            const int v = base + lane;
-            const bool valid = v < L;
-            const int vv = valid ? v : L - 1;
-            int q = 0;
-#pragma unroll
-            for (int st = 16; st > 0; st >>= 1)
-                if (sh_vst[w][q + st] <= vv) q += st;
-            const int off = vv - sh_vst[w][q];
-            const int j = sh_rj[w][q] + off;
-            const int s = sh_rs[w][q] + off;
-            const float4 xj4 = staged ? stage[s] : __ldg(D.xm + j);
-            const float3 xj = f3(xj4);
-            const int jr = j - pb;
-#pragma unroll
-            for (int p = 0; p < PP; ++p) {
-                if (p < np) {
-                    const bool hit = valid && jr != p && norm2_rn(sub3(xi[p], xj)) <= r2max;
-                    const unsigned ball = __ballot_sync(0xffffffffu, hit);
-                    const int pos = cnt[p] + __popc(ball & lt);
-                    if (hit && pos < cap) {
-                        hit_j[w][p][pos] = j;
-                        hit_s[w][p][pos] = (short)s;
-                    }
-                    cnt[p] += __popc(ball);
-                }
-            }
-        }
-        __syncwarp();
-        // phase 2: dense over the hits, LPP lanes per particle
-        const int p = lane / LPP, sub = lane % LPP;
-        int found = 0;
-#pragma unroll
-        for (int t = 0; t < PP; ++t)
-            if (t == p) found = cnt[t];
-        const bool act = p < np;
-        const int n_hit = act ? min(found, cap) : 0;
-        const int i = pb + (act ? p : 0);
-        const float4 xi4 = D.xm[i];
-        const float3 xs = f3(xi4);
-        const int row = P.row_base + (i - P.s_begin);
-        float4* out = D.nbr + (size_t)row * D.stride;
-        float2* out2 = reinterpret_cast<float2*>(D.nbr) + (size_t)row * D.stride;
-        float rho = 0.0f, aii = 0.0f;
-        float3 jii = make_float3(0.0f, 0.0f, 0.0f);
-        for (int kk = sub; kk < n_hit; kk += LPP) {
-            const int j = hit_j[w][p][kk];
-            const float4 xj4 = staged ? stage[hit_s[w][p][kk]] : __ldg(D.xm + j);
-            const float3 r = sub3(xs, f3(xj4));
-            // spiky gradient (sph_kernel.py:52-61): -k (h - |r|)^2 r / |r|
-            const float rn = sqrtf(norm2_rn(r));
-            const float rc = rn < 1e-6f ? 1e-6f : rn;
-            const float t = h - rc;
-            const float sg = -spk * (t * t);
-            const float ir = __frcp_rn(rc);
-            const float mj = xj4.w;
-            const float wgt = mj * (sg * ir);
-            const float3 J = make_float3(__fmul_rn(wgt, r.x), __fmul_rn(wgt, r.y), __fmul_rn(wgt, r.z));
-            if (D.row_fmt == ROW_FULL) {
-                out[kk] = make_float4(J.x, J.y, J.z, __int_as_float(j));
-            } else if (D.row_fmt == ROW_COMPACT) {
-                out2[kk] = make_float2(__int_as_float(j), wgt);
-            } else {
-                const size_t e = (size_t)row * D.stride + kk;
-                reinterpret_cast<int*>(D.nbr)[e] = j;
-                unsigned short* gb = D.nbr_g + 3 * e;
-                gb[0] = bf16_bits(J.x);
-                gb[1] = bf16_bits(J.y);
-                gb[2] = bf16_bits(J.z);
-            }
-            rho += mj * cubic_Wq(rn * inv_h, ck);
-            if (j < dyn_end) aii += dot3(J, J) * __frcp_rn(mj);
-            jii = sub3(jii, J);
-        }
-#pragma unroll
-        for (int o = LPP / 2; o > 0; o >>= 1) {
-            rho += __shfl_xor_sync(0xffffffffu, rho, o);
-            aii += __shfl_xor_sync(0xffffffffu, aii, o);
-            jii.x += __shfl_xor_sync(0xffffffffu, jii.x, o);
-            jii.y += __shfl_xor_sync(0xffffffffu, jii.y, o);
-            jii.z += __shfl_xor_sync(0xffffffffu, jii.z, o);
-        }
-        if (act && sub == 0) {
-            const float mi = xi4.w;
-            float dens = 0.0f;
-            dens = dens + mi * P.W0;
-            dens += rho;
-            aii += dot3(jii, jii) * __frcp_rn(mi);
-            const float kd = __frcp_rn(aii + 1e-3f);
-            D.nbr_cnt[row] = n_hit;
-            D.dens[i] = dens;
-            D.kd[i] = kd;
-            D.c[i] = dens - D.rho0s[i];
-            const int pid = D.pid[i];
-            D.rflu[i] = D.material[pid] == 1 ? __frcp_rn(dens) : 0.0f;
-            D.density_out[pid] = dens;
-            D.k_out[pid] = kd;
-            if (found > cap) {
-                // truncated list: the fix-up rebuilds the row in the
-                // reference's candidate order and adds transpose corrections
-                atomicAdd(&D.overflow[sc], 1);
-                D.ovf_list[atomicAdd(&D.ovf_ctr[0], 1)] = i;
-                set_cond(D.h_fix, 1u);
-            }
-            my_pairs += n_hit;
-        }
-        __syncwarp();
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) my_pairs += __shfl_xor_sync(0xffffffffu, my_pairs, o);
-    if (lane == 0 && my_pairs) atomicAdd(&sh_pairs, my_pairs);
-    __syncthreads();
-    if (threadIdx.x == 0 && sh_pairs) atomicAdd(&D.pairs[sc], (unsigned long long)sh_pairs);
+    __syncwarp();
+    const int n_hit = min(found, cap);
+    for (int k = lane; k < n_hit; k += 32) {
+        const int j = list[k];
+        const float4 xj = __ldg(W.xm + j);
+        const float3 r = make_float3(xi.x - xj.x, xi.y - xj.y, xi.z - xj.z);
+        float w;
+        const float3 J = hit_terms(r, norm2_rn(r), xj.w, j < dyn_end, h, inv_h, spk, ck, s, &w);
+        entry(k, j, J, w);
+    }
+    sum_lanes<32>(s);
+    __syncwarp();
+    return found;
+}
+
+template <int SUB>
+__global__ void __launch_bounds__(32 * kBuildWarps) k_nbr_build(const Dev D, int tile_size) {
+    __shared__ BuildShared<SUB> sh[kBuildWarps];
+    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    BuildShared<SUB>& S = sh[wid];
+    const int per_tile = (tile_size + SUB - 1) / SUB;
+    const int gw = blockIdx.x * kBuildWarps + wid;
+    const int t = gw / per_tile;
+    if (t >= D.n_tiles) return;  // warp-uniform; the kernel has no CTA barrier
+    const int4 tile = __ldg(D.tiles + t);
+    const int i0 = tile.y + (gw - t * per_tile) * SUB;
+    const int n = min(SUB, tile.z - i0);
+    if (n <= 0) return;
+    const int sc = tile.x;
+    const SceneParams& P = D.scenes[sc];
+    WindowGrid W;
+    W.cell_start = D.cell_start + P.key_base;
+    W.xm = D.xm;
+    W.ncell = P.ncell;
+    W.dims[0] = P.dims[0];
+    W.dims[1] = P.dims[1];
+    W.dims[2] = P.dims[2];
+    W.r2_max = P.r2_max;
+    const int cap = min(min(P.cache, D.stride), kHits);
+    const int dyn_end = P.s_dyn_end;
+    const float h = P.h, inv_h = P.inv_h, spk = P.spiky_k, ck = P.cubic_k;
+    auto cell_of = [&](float4 x) {
+        return make_int3(cell_coord(x.x, P.cell_inv, W.dims[0]), cell_coord(x.y, P.cell_inv, W.dims[1]),
+                         cell_coord(x.z, P.cell_inv, W.dims[2]));
+    };
+    float4 xl = make_float4(0.f, 0.f, 0.f, 0.f);
+    int3 cell = make_int3(0, 0, 0);
+    int pid = 0, material = 0;
+    float rho0 = 0.0f;
+    if (lane < n) {
+        // what the last lines need comes with the first loads
+        xl = __ldg(D.xm + i0 + lane);
+        pid = D.pid[i0 + lane];
+        rho0 = D.rho0s[i0 + lane];
+        cell = cell_of(xl);
+        material = D.material[pid];
+    }
+    const int mine = filter_hits<SUB>(W, S, i0, n, xl, cell, cap);
+    __syncwarp();
+    // the row entry, density and Aii terms of hit k of slot i
+    auto take = [&](int i, int k, int j, float4 xi, float4 xj, float3 r, float r2, HitSums& s) {
+        float w;
+        const float3 J = hit_terms(r, r2, xj.w, j < dyn_end, h, inv_h, spk, ck, s, &w);
+        put_entry(D, P.row_base + (i - P.s_begin), k, j, J, w);
+    };
+    HitSums s;      // lane p's own particle
+    int found = lane < n ? S.found[lane] : 0;
+    const unsigned alone = __ballot_sync(0xffffffffu, found < 0);
+    {
+        // eight lanes per particle, four particles at a time
+        const int sub = lane & 7;
+        for (int p0 = 0; p0 < n; p0 += 4) {
+            const int p = p0 + (lane >> 3);
+            const int n_hit = p < n ? min(S.found[p], cap) : 0;
+            const int* delta = S.delta[__shfl_sync(0xffffffffu, mine, min(p, n - 1))];
+            const float4 xi = S.pos[min(p, n - 1)];
+            HitSums a;
+            for (int k = sub; k < n_hit; k += 8) {
+                const int code = S.hit[k][p];
+                const int j = delta[code >> kOrdShift] + (code & ((1 << kOrdShift) - 1));
+                const float4 xj = __ldg(D.xm + j);
+                const float3 r = make_float3(xi.x - xj.x, xi.y - xj.y, xi.z - xj.z);
+                take(i0 + p, k, j, xi, xj, r, norm2_rn(r), a);
+            }
+            __syncwarp();
+            sum_lanes<8>(a);
+            own_sums(a, p0, s);
+        }
+    }
+    __syncwarp();
+    for (unsigned left = alone; left; left &= left - 1u) {
+        const int q = __ffs(left) - 1;
+        const float4 xq = S.pos[q];
+        const int rq = P.row_base + (i0 + q - P.s_begin);
+        HitSums a;
+        const int f = scan_alone(W, reinterpret_cast<int*>(S.mask), i0 + q, xq, cell_of(xq), cap, dyn_end, h, inv_h,
+                                 spk, ck, a, [&](int k, int j, float3 J, float w) { put_entry(D, rq, k, j, J, w); });
+        if (lane == q) {
+            s = a;
+            found = f;
+        }
+    }
+    // every row of a slice up to the slice's widest
+    const bool act = lane < n;
+    const int i = i0 + (act ? lane : 0), row = P.row_base + (i - P.s_begin);
+    int pairs = act ? min(found, cap) : 0;
+    int widest = pairs;
+    for (int o = 1; o < (32 >> D.lg); o <<= 1) widest = max(widest, __shfl_xor_sync(0xffffffffu, widest, o));
+    if (act) {
+        put_pads(D, row, pairs, slice_entries(D, widest), i, 0, 1);
+        const float mi = xl.w;
+        float dens = 0.0f;
+        dens = dens + mi * P.W0;
+        dens += s.rho;
+        const float aii = s.aii + dot3(s.jii, s.jii) * __frcp_rn(mi);
+        const float kd = __frcp_rn(aii + 1e-3f);
+        D.nbr_cnt[row] = pairs;
+        D.dens[i] = dens;
+        D.kd[i] = kd;
+        D.c[i] = dens - rho0;
+        D.rflu[i] = material == 1 ? __frcp_rn(dens) : 0.0f;
+        D.density_out[pid] = dens;
+        D.k_out[pid] = kd;
+        if (found > cap) {
+            // truncated list: the fix-up rebuilds the row in the
+            // reference's candidate order and adds transpose corrections
+            atomicAdd(&D.overflow[sc], 1);
+            D.ovf_list[atomicAdd(&D.ovf_ctr[0], 1)] = i;
+            set_cond(D.h_fix, 1u);
+        }
+    }
+    pairs = __reduce_add_sync(0xffffffffu, pairs);
+    if (lane == 0 && pairs) atomicAdd(&D.pairs[sc], (unsigned long long)pairs);
 }
 
 // Neighbour lists, density, Aii, k, c and 1/rho of every dynamic particle,
@@ -812,8 +715,6 @@ __global__ void __launch_bounds__(kTppMaxThreads) k_nbr_build_tpp(const Dev D) {
         const float h = P.h, inv_h = P.inv_h, spk = P.spiky_k, ck = P.cubic_k;
         const int dyn_end = P.s_dyn_end;
         const int row = P.row_base + (i - P.s_begin);
-        float4* out = D.nbr + (size_t)row * D.stride;
-        float2* out2 = reinterpret_cast<float2*>(D.nbr) + (size_t)row * D.stride;
         float rho = 0.0f, aii = 0.0f;
         float3 jii = make_float3(0.0f, 0.0f, 0.0f);
         int q_cur = -1, jb_cur = 0;
@@ -852,18 +753,7 @@ __global__ void __launch_bounds__(kTppMaxThreads) k_nbr_build_tpp(const Dev D) {
                 const float mj = xj4.w;
                 const float wgt = mj * (sg * ir);
                 const float3 J = make_float3(__fmul_rn(wgt, r.x), __fmul_rn(wgt, r.y), __fmul_rn(wgt, r.z));
-                if (D.row_fmt == ROW_FULL) {
-                    out[k] = make_float4(J.x, J.y, J.z, __int_as_float(j));
-                } else if (D.row_fmt == ROW_COMPACT) {
-                    out2[k] = make_float2(__int_as_float(j), wgt);
-                } else {
-                    const size_t e = (size_t)row * D.stride + k;
-                    reinterpret_cast<int*>(D.nbr)[e] = j;
-                    unsigned short* gb = D.nbr_g + 3 * e;
-                    gb[0] = bf16_bits(J.x);
-                    gb[1] = bf16_bits(J.y);
-                    gb[2] = bf16_bits(J.z);
-                }
+                put_entry(D, row, k, j, J, wgt);
                 rho += mj * cubic_Wq(rn * inv_h, ck);
                 if (j < dyn_end) aii += dot3(J, J) * __frcp_rn(mj);
                 jii = sub3(jii, J);
@@ -889,6 +779,10 @@ __global__ void __launch_bounds__(kTppMaxThreads) k_nbr_build_tpp(const Dev D) {
             set_cond(D.h_fix, 1u);
         }
     }
+    // every row of a slice up to the slice's widest
+    int widest = n_hit;
+    for (int o = 1; o < (32 >> D.lg); o <<= 1) widest = max(widest, __shfl_xor_sync(0xffffffffu, widest, o));
+    if (act) put_pads(D, P.row_base + (i - P.s_begin), n_hit, slice_entries(D, widest), i, 0, 1);
     // pair count of the scene (a tile never spans scenes): one atomic per CTA
     int pairs = n_hit;
 #pragma unroll
@@ -977,8 +871,6 @@ __global__ void __launch_bounds__(256) k_ovf_rows(const Dev D) {
         }
         const int cap = min(min(P.cache, D.stride), 64);
         const int row = P.row_base + (i - P.s_begin);
-        float4* out = D.nbr + (size_t)row * D.stride;
-        float2* out2 = reinterpret_cast<float2*>(D.nbr) + (size_t)row * D.stride;
         float rho = 0.0f, aii = 0.0f;
         float3 jii = make_float3(0.0f, 0.0f, 0.0f);
         for (int h = lane; h < H; h += 32) {
@@ -1005,18 +897,7 @@ __global__ void __launch_bounds__(256) k_ovf_rows(const Dev D) {
             const float mj = xj4.w;
             const float wgt = mj * (sg * ir);
             const float3 J = make_float3(__fmul_rn(wgt, rv.x), __fmul_rn(wgt, rv.y), __fmul_rn(wgt, rv.z));
-            if (D.row_fmt == ROW_FULL) {
-                out[r] = make_float4(J.x, J.y, J.z, __int_as_float(j));
-            } else if (D.row_fmt == ROW_COMPACT) {
-                out2[r] = make_float2(__int_as_float(j), wgt);
-            } else {
-                const size_t e = (size_t)row * D.stride + r;
-                reinterpret_cast<int*>(D.nbr)[e] = j;
-                unsigned short* gb = D.nbr_g + 3 * e;
-                gb[0] = bf16_bits(J.x);
-                gb[1] = bf16_bits(J.y);
-                gb[2] = bf16_bits(J.z);
-            }
+            put_entry(D, row, r, j, J, wgt);
             rho += mj * cubic_Wq(rn * P.inv_h, P.cubic_k);
             if (j < P.s_dyn_end) aii += dot3(J, J) * __frcp_rn(mj);
             jii = sub3(jii, J);
@@ -1149,8 +1030,7 @@ __global__ void __launch_bounds__(BLOCK) k_density(const Dev D) {
     }
     float acc = 0.0f;
     for (int k = lane; k < cnt; k += G) {
-        const int j = row_j(D, row, k);
-        const int pj = D.pid[j];
+        const int pj = D.pid[row_j(D, row, k)];
         const float3 r = sub3(xi, make_float3(D.x[3 * pj], D.x[3 * pj + 1], D.x[3 * pj + 2]));
         acc += D.m[pj] * cubic_W(sqrtf(dot3(r, r)), P.h, P.cubic_k);
     }
@@ -1315,18 +1195,9 @@ __global__ void k_advect(const Dev D) {
 // k_advect with advect_skip_failed.
 __global__ void k_advect_keys(const Dev D) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    // the build's per-scene counters start from zero (read from k_place on)
-    if (p < D.n_scenes) {
-        D.overflow[p] = 0;
-        D.pairs[p] = 0ull;
-        D.fix_fail[p] = 0;
-        D.fix_scene[p] = 0;
-    }
-    if (p == 0) {
-        D.seg_ctr[0] = 0;
-        D.ovf_ctr[0] = 0;
-        D.ovf_ctr[1] = 0;
-    }
+    build_begin(D, p);
+    // the solves of the step are over: their barrier counters go back to zero
+    if (p < kBarrierWords) D.bar_count[p] = 0u;
     if (p >= D.n_total) return;
     const int sc = D.pscene[p];
     float pos[3];
@@ -1342,123 +1213,88 @@ __global__ void k_advect_keys(const Dev D) {
 
 // ------------------------------------------------------------- IP solve
 
-// Pair-loop unroll: each lane loads PU list entries before gathering, so PU
-// independent gather chains are in flight.  The entries come in 32-byte
-// pairs: in a batch of G * PU entries starting at a multiple of G * PU, lane
-// l takes entries 2l + 2Gu and 2l + 2Gu + 1 (u < PU / 2), one 256-bit load
-// each.  Rows start on 1 KB boundaries and the list stride is even, so the
-// second entry of a pair is inside the row whenever the first is below the
-// count.  Entries past the row end become (self, w = 0), which contributes
-// exactly 0; entries outside the scene are redirected to self and reported
-// once after the loop.
-#ifndef IVP_PAIR_UNROLL
-#define IVP_PAIR_UNROLL 4
-#endif
-constexpr int PU = IVP_PAIR_UNROLL;
-static_assert(PU % 2 == 0, "entries are loaded in pairs");
-
+// N list entries of one lane, whose loads and gathers are in flight together.
+template <int N_>
 struct PairBatch {
-    int j[PU];
-    float3 J[PU];
-    unsigned live;  // bit u: entry u is a neighbour (not a masked slot past the row end)
+    static constexpr int N = N_;
+    int j[N];
+    float3 J[N];
 };
 
-__device__ __forceinline__ void pair_entry(const float4& e, bool in, int self, int lo, int hi, int& j, float3& J,
-                                           bool& bad, unsigned& live, int u) {
-    const int jj = __float_as_int(e.w);
-    const bool ok = jj >= lo && jj < hi;
-    bad |= in && !ok;
-    j = (in && ok) ? jj : self;
-    J = (in && ok) ? f3(e) : make_float3(0.f, 0.f, 0.f);
-    live |= (in && ok) ? (1u << u) : 0u;
-}
+// The reader of a tile's rows.
+template <int G, int F>
+struct Rows {
+    const Dev& D;
+    int cnt = 0;
+    __device__ __forceinline__ explicit Rows(const Dev& d) : D(d) {}
+    // the tile's own row
+    __device__ __forceinline__ void open(int row, bool valid) { cnt = valid ? D.nbr_cnt[row] : 0; }
 
-// k0 = 2 * lane + (batch start); xi is the row particle's position (the
-// compact rows recompute J_ij = w_ij (x_i - x_j) from it).
-template <int G>
-__device__ __forceinline__ bool load_pairs(const Dev& D, int row, float3 xi, int k0, int cnt, int self, int lo,
-                                           int hi, PairBatch& b) {
-    bool bad = false;
-    b.live = 0u;
-    if (D.row_fmt == ROW_BF16) {
-        // entries k, k+1 (k even): ids as one 8-byte load, gradients as
-        // three 4-byte words of bf16 pairs
-        const int2* __restrict__ ids = reinterpret_cast<const int2*>(reinterpret_cast<const int*>(D.nbr) +
-                                                                     (size_t)row * D.stride);
-        const unsigned* __restrict__ gw =
-            reinterpret_cast<const unsigned*>(D.nbr_g + 3 * (size_t)row * D.stride);
+    // The lane's N entries from list entry e on.
+    template <int N>
+    __device__ __forceinline__ PairBatch<N> load(size_t e, float3 xi) const {
+        PairBatch<N> b;
+        if (F != READ_ANY || D.row_fmt == ROW_FULL) {
+            float4 q[N];
 #pragma unroll
-        for (int u = 0; u < PU / 2; ++u) {
-            const int k = k0 + u * 2 * G;
-            int2 jj = make_int2(self, self);
-            unsigned w0 = 0u, w1 = 0u, w2 = 0u;
-            if (k < cnt) {
-                jj = __ldg(ids + (k >> 1));
-                const unsigned* p = gw + (3 * k >> 1);
-                w0 = __ldg(p);
-                w1 = __ldg(p + 1);
-                w2 = __ldg(p + 2);
+            for (int u = 0; u < N; u += 2) {
+                const float4* p = D.nbr + e + lane_entry(u);
+                if (F == READ_STREAM || (F == READ_ANY && D.row_stream)) ld_rec_nc_stream(p, q[u], q[u + 1]);
+                else ld_rec_nc(p, q[u], q[u + 1]);
             }
-            const float4 e0 = make_float4(bf16_lo(w0), bf16_hi(w0), bf16_lo(w1), __int_as_float(jj.x));
-            const float4 e1 = make_float4(bf16_hi(w1), bf16_lo(w2), bf16_hi(w2), __int_as_float(jj.y));
-            pair_entry(e0, k < cnt, self, lo, hi, b.j[2 * u], b.J[2 * u], bad, b.live, 2 * u);
-            pair_entry(e1, k + 1 < cnt, self, lo, hi, b.j[2 * u + 1], b.J[2 * u + 1], bad, b.live, 2 * u + 1);
-        }
-    } else if (D.row_fmt == ROW_FULL) {
-        const float4* __restrict__ nb = D.nbr + (size_t)row * D.stride;
 #pragma unroll
-        for (int u = 0; u < PU / 2; ++u) {
-            const int k = k0 + u * 2 * G;
-            float4 e0 = make_float4(0.f, 0.f, 0.f, 0.f), e1 = e0;
-            if (k < cnt) {
-                if (D.row_stream) ld_rec_nc_stream(nb + k, e0, e1);
-                else ld_rec_nc(nb + k, e0, e1);
+            for (int u = 0; u < N; ++u) {
+                b.j[u] = __float_as_int(q[u].w);
+                b.J[u] = f3(q[u]);
             }
-            pair_entry(e0, k < cnt, self, lo, hi, b.j[2 * u], b.J[2 * u], bad, b.live, 2 * u);
-            pair_entry(e1, k + 1 < cnt, self, lo, hi, b.j[2 * u + 1], b.J[2 * u + 1], bad, b.live, 2 * u + 1);
-        }
-    } else {
-        const float4* __restrict__ nb =
-            reinterpret_cast<const float4*>(reinterpret_cast<const float2*>(D.nbr) + (size_t)row * D.stride);
+        } else if (D.row_fmt == ROW_COMPACT) {
+            // {j, w, j, w}; J_ij = w_ij (x_i - x_j)
+            float w[N];
 #pragma unroll
-        for (int u = 0; u < PU / 2; ++u) {
-            const int k = k0 + u * 2 * G;
-            float4 e = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (k < cnt) e = __ldg(nb + (k >> 1));  // entries k, k+1: {j, w, j, w}
+            for (int u = 0; u < N; u += 2) {
+                const float4 v = __ldg(
+                    reinterpret_cast<const float4*>(reinterpret_cast<const float2*>(D.nbr) + e + lane_entry(u)));
+                b.j[u] = __float_as_int(v.x);
+                w[u] = v.y;
+                b.j[u + 1] = __float_as_int(v.z);
+                w[u + 1] = v.w;
+            }
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int jj = __float_as_int(h ? e.z : e.x);
-                const float w = h ? e.w : e.y;
-                const bool in = k + h < cnt;
-                const bool ok = jj >= lo && jj < hi;
-                bad |= in && !ok;
-                const int j = (in && ok) ? jj : self;
-                const float3 r = sub3(xi, f3(__ldg(D.xm + j)));
-                b.j[2 * u + h] = j;
-                b.live |= (in && ok) ? (1u << (2 * u + h)) : 0u;
-                b.J[2 * u + h] = (in && ok) ? make_float3(__fmul_rn(w, r.x), __fmul_rn(w, r.y), __fmul_rn(w, r.z))
-                                            : make_float3(0.f, 0.f, 0.f);
+            for (int u = 0; u < N; ++u) {
+                const float3 r = sub3(xi, f3(__ldg(D.xm + b.j[u])));
+                b.J[u] = make_float3(__fmul_rn(w[u], r.x), __fmul_rn(w[u], r.y), __fmul_rn(w[u], r.z));
+            }
+        } else {
+            // ids as 8-byte loads, gradients as three 4-byte words of bf16 pairs
+#pragma unroll
+            for (int u = 0; u < N; u += 2) {
+                const size_t k = e + lane_entry(u);
+                const int2 jj = __ldg(reinterpret_cast<const int2*>(reinterpret_cast<const int*>(D.nbr) + k));
+                const unsigned* gw = reinterpret_cast<const unsigned*>(D.nbr_g + 3 * k);
+                const unsigned w0 = __ldg(gw), w1 = __ldg(gw + 1), w2 = __ldg(gw + 2);
+                b.j[u] = jj.x;
+                b.J[u] = make_float3(bf16_lo(w0), bf16_hi(w0), bf16_lo(w1));
+                b.j[u + 1] = jj.y;
+                b.J[u + 1] = make_float3(bf16_hi(w1), bf16_lo(w2), bf16_hi(w2));
             }
         }
+        return b;
     }
-    return bad;
-}
 
-// The pair loop of one row: batches of PU entries per lane, `body(b)`
-// consuming one batch.  (Requesting batch k+1's entries before batch k's
-// gathers spills at the persistent kernels' 64-register budget and measured
-// 20-35 % slower.)
-template <int G, class Body>
-__device__ __forceinline__ bool pair_loop(const Dev& D, int row, float3 xi, int cnt, int lane, int self, int lo,
-                                          int hi, Body&& body) {
-    bool bad = false;
-    for (int k0 = 2 * lane; k0 < cnt; k0 += G * PU) {
-        PairBatch b;
-        bad |= load_pairs<G>(D, row, xi, k0, cnt, self, lo, hi, b);
-        body(b);
+    // `body(b, k, e)` consumes the row in batches of four entries a lane (two at
+    // the end): list positions k, k + 1, k + 2 G, k + 2 G + 1, at entries
+    // e + lane_entry(u) of the list arrays.  The build filled up the row's last
+    // pairs (put_pads) and wrote every index, so an entry costs its loads and
+    // its arithmetic.
+    template <class Body>
+    __device__ __forceinline__ void each(int row, float3 xi, Body&& body) {
+        const int lane = threadIdx.x & 31;
+        size_t e = (size_t)(row - lane / G) * D.stride + 2 * lane;
+        int k = 0;
+        for (; k + 2 * G < cnt; k += 4 * G, e += lane_entry(4)) body(load<4>(e, xi), k + 2 * (lane % G), e);
+        if (k < cnt) body(load<2>(e, xi), k + 2 * (lane % G), e);
     }
-    return bad;
-}
+};
 
 // Shared prologue of the neighbour-sum kernels: tile, scene, particle.
 struct TileCtx {
@@ -1491,8 +1327,8 @@ __device__ __forceinline__ void pf_l1(const void* p) { asm volatile("prefetch.gl
 // (pressure_base.py:187-203), with the previous outer update d -= sol
 // (ip.py:389) applied on the fly (it = updates applied so far).  Writes
 // s = dfdt k and fk = f k for the rhs and CG phases.
-template <int G>
-__device__ __forceinline__ double pack_tile(const Dev& D, const SceneParams& P, const TileCtx& T, int it) {
+template <int G, class R>
+__device__ __forceinline__ double pack_tile(R& rows, const Dev& D, const SceneParams& P, const TileCtx& T, int it) {
     const bool upd = it >= 1;
     const float4* src = (upd && ((it - 1) & 1)) ? D.d1 : D.d0;
     float4* dst = (it & 1) ? D.d1 : D.d0;
@@ -1505,29 +1341,25 @@ __device__ __forceinline__ double pack_tile(const Dev& D, const SceneParams& P, 
         pf_l1(D.inv_m + T.i);
         pf_l1(D.rho0s + T.i);
     }
-    const int cnt = T.valid ? D.nbr_cnt[T.row] : 0;
     float3 xi = make_float3(0.f, 0.f, 0.f), di = xi;
     if (T.valid) {
         xi = f3(D.xm[T.i]);
         di = f3(dsrc[T.i]);
     }
     float acc = 0.0f;
-    bool bad = false;
-    const int self = T.valid ? T.i : P.s_begin;
-    for (int k0 = 2 * T.lane; k0 < cnt; k0 += G * PU) {
-        PairBatch b;
-        bad |= load_pairs<G>(D, T.row, xi, k0, cnt, self, P.s_begin, P.s_end, b);
+    rows.open(T.row, T.valid);
+    rows.each(T.row, xi, [&](const auto& b, int, size_t) {
 #pragma unroll
-        for (int u = 0; u < PU; ++u) {
+        for (int u = 0; u < b.N; ++u) {
             const float3 dj = f3(dsrc[b.j[u]]);
             acc += dot3(sub3(di, dj), b.J[u]);
         }
-    }
-    if (bad) flag_bad(D, T.i, 1);
+    });
     acc = group_sum<G>(acc);
     double part = 0.0;
     if (T.valid && T.lane == 0) {
         if (upd) dst[T.i] = make_float4(di.x, di.y, di.z, 0.0f);
+        if (D.div_out) D.jd[T.i] = acc;
         const float t = acc + D.c[T.i];
         const float f = t > 0.0f ? t : 0.0f;
         const float kd = D.kd[T.i];
@@ -1544,10 +1376,9 @@ __device__ __forceinline__ double pack_tile(const Dev& D, const SceneParams& P, 
 
 // ip_rhs_fused (ip.py:174-215) fused with the CG start: sol = 0 (ip.py:384),
 // r = rhs, p_prev = 0, rr = r.r (ip.py:293-296).
-template <int G>
-__device__ __forceinline__ double rhs_tile(const Dev& D, const SceneParams& P, const TileCtx& T,
+template <int G, class R>
+__device__ __forceinline__ double rhs_tile(R& rows, const Dev& D, const SceneParams& P, const TileCtx& T,
                                            const float4* __restrict__ dcur) {
-    const int cnt = T.valid ? D.nbr_cnt[T.row] : 0;
     float3 xi = make_float3(0.f, 0.f, 0.f);
     float fki = 0.0f, mi = 0.0f;
     if (T.valid) {
@@ -1557,20 +1388,16 @@ __device__ __forceinline__ double rhs_tile(const Dev& D, const SceneParams& P, c
         fki = D.fk[T.i];
     }
     float ax = 0.0f, ay = 0.0f, az = 0.0f;
-    bool bad = false;
-    const int self = T.valid ? T.i : P.s_begin;
-    for (int k0 = 2 * T.lane; k0 < cnt; k0 += G * PU) {
-        PairBatch b;
-        bad |= load_pairs<G>(D, T.row, xi, k0, cnt, self, P.s_begin, P.s_end, b);
+    rows.open(T.row, T.valid);
+    rows.each(T.row, xi, [&](const auto& b, int, size_t) {
 #pragma unroll
-        for (int u = 0; u < PU; ++u) {
+        for (int u = 0; u < b.N; ++u) {
             const float wgt = fki + mi * D.q[b.j[u]];
             ax += wgt * b.J[u].x;
             ay += wgt * b.J[u].y;
             az += wgt * b.J[u].z;
         }
-    }
-    if (bad) flag_bad(D, T.i, 2);
+    });
     ax = group_sum<G>(ax);
     ay = group_sum<G>(ay);
     az = group_sum<G>(az);
@@ -1596,8 +1423,8 @@ __device__ __forceinline__ double rhs_tile(const Dev& D, const SceneParams& P, c
 // the next iteration.  y = dfdt k (J p), and the FP64 partials of
 // p^T A p = sum m |p|^2 + omega sum y (J p) (the value dot(p, A p) of
 // ip.py:307: phase B applies the exact transpose of J).
-template <int G>
-__device__ __forceinline__ double cga_tile(const Dev& D, const SceneParams& P, const TileCtx& T, float beta,
+template <int G, class R>
+__device__ __forceinline__ double cga_tile(R& rows, const Dev& D, const SceneParams& P, const TileCtx& T, float beta,
                                            int cg_it) {
     if (T.valid && T.lane == 0) {
         pf_l1(D.pip + T.i);
@@ -1605,22 +1432,20 @@ __device__ __forceinline__ double cga_tile(const Dev& D, const SceneParams& P, c
         pf_l1(D.s + T.i);
         pf_l1(D.inv_m + T.i);
     }
-    const int cnt = T.valid ? D.nbr_cnt[T.row] : 0;
     float3 xi = make_float3(0.f, 0.f, 0.f), ri = xi;
     if (T.valid) {
         xi = f3(D.xm[T.i]);
         ri = f3(D.rip[T.i]);
     }
     float acc = 0.0f;
-    const int self = T.valid ? T.i : P.s_begin;
-    const bool bad = pair_loop<G>(D, T.row, xi, cnt, T.lane, self, P.s_begin, P.s_end, [&](const PairBatch& b) {
+    rows.open(T.row, T.valid);
+    rows.each(T.row, xi, [&](const auto& b, int, size_t) {
 #pragma unroll
-        for (int u = 0; u < PU; ++u) {
+        for (int u = 0; u < b.N; ++u) {
             const float3 rj = f3(ld_vec(D.rip + b.j[u]));
             acc += dot3(sub3(ri, rj), b.J[u]);
         }
     });
-    if (bad) flag_bad(D, T.i, 3);
     acc = group_sum<G>(acc);
     double part = 0.0;
     if (T.valid && T.lane == 0) {
@@ -1658,8 +1483,8 @@ __device__ __noinline__ float3 ovf_correction(const int* __restrict__ fix_off, c
 // CG phase B: Ap = m p + omega J^T y in gather form (compute_Ax_part1/2,
 // ip.py:63-121, as pressure_base.py:130-166 writes J^T), x += alpha p,
 // r -= alpha Ap (pcg_update_x_r_scalar, math_utils.py:181-195), rr = r.r.
-template <int G>
-__device__ __forceinline__ double cgb_tile(const Dev& D, const SceneParams& P, const TileCtx& T, float alpha,
+template <int G, class R>
+__device__ __forceinline__ double cgb_tile(R& rows, const Dev& D, const SceneParams& P, const TileCtx& T, float alpha,
                                            int cg_it, const float4* __restrict__ dcur) {
     if (T.valid && T.lane == 0) {
         pf_l1(D.pip + T.i);
@@ -1667,7 +1492,6 @@ __device__ __forceinline__ double cgb_tile(const Dev& D, const SceneParams& P, c
         pf_l1(D.rip + T.i);
         pf_l1(dcur + T.i);
     }
-    const int cnt = T.valid ? D.nbr_cnt[T.row] : 0;
     float3 xi = make_float3(0.f, 0.f, 0.f);
     float mi = 0.0f, yi = 0.0f;
     if (T.valid) {
@@ -1677,17 +1501,16 @@ __device__ __forceinline__ double cgb_tile(const Dev& D, const SceneParams& P, c
         yi = D.y[T.i];
     }
     float ax = 0.0f, ay = 0.0f, az = 0.0f;
-    const int self = T.valid ? T.i : P.s_begin;
-    const bool bad = pair_loop<G>(D, T.row, xi, cnt, T.lane, self, P.s_begin, P.s_end, [&](const PairBatch& b) {
+    rows.open(T.row, T.valid);
+    rows.each(T.row, xi, [&](const auto& b, int, size_t) {
 #pragma unroll
-        for (int u = 0; u < PU; ++u) {
+        for (int u = 0; u < b.N; ++u) {
             const float wgt = yi + mi * D.z[b.j[u]];
             ax += wgt * b.J[u].x;
             ay += wgt * b.J[u].y;
             az += wgt * b.J[u].z;
         }
     });
-    if (bad) flag_bad(D, T.i, 4);
     ax = group_sum<G>(ax);
     ay = group_sum<G>(ay);
     az = group_sum<G>(az);
@@ -1720,11 +1543,19 @@ __device__ __forceinline__ double cgb_tile(const Dev& D, const SceneParams& P, c
     return part;
 }
 
-// compute_divergence (pressure_base.py:449-457): max(J v, 0) with v = d/dt.
-template <int G>
-__device__ __forceinline__ void div_tile(const Dev& D, const SceneParams& P, const TileCtx& T, int outer_it) {
-    const float4* dc = (outer_it & 1) ? D.d1 : D.d0;
-    const int cnt = T.valid ? D.nbr_cnt[T.row] : 0;
+// compute_divergence (pressure_base.py:449-457): max(J v, 0) with v = d/dt.  The
+// last pack (or PRJ tail) of a solve formed J d at the final d, so the neighbours
+// are summed here only for a scene that was stopped before its first one.
+template <int G, class R>
+__device__ __forceinline__ void div_tile(R& rows, const Dev& D, const SceneParams& P, const TileCtx& T, const SceneCtl& C) {
+    if (C.n_err > 0) {
+        if (T.valid && T.lane == 0) {
+            const float dv = P.inv_dt * D.jd[T.i];
+            D.div_out[D.pid[T.i]] = dv > 0.0f ? dv : 0.0f;
+        }
+        return;
+    }
+    const float4* dc = D.d0;
     const float s = P.inv_dt;
     float3 xi = make_float3(0.f, 0.f, 0.f), vi = xi;
     if (T.valid) {
@@ -1732,14 +1563,13 @@ __device__ __forceinline__ void div_tile(const Dev& D, const SceneParams& P, con
         vi = scale3(s, f3(dc[T.i]));
     }
     float acc = 0.0f;
-    for (int k = T.lane; k < cnt; k += G) {
-        int j;
-        const float3 J = row_J(D, T.row, k, xi, &j);
-        const float3 vj = scale3(s, f3(dc[j]));
-        acc += dot3(sub3(vi, vj), J);
-    }
+    rows.open(T.row, T.valid);
+    rows.each(T.row, xi, [&](const auto& b, int, size_t) {
+#pragma unroll
+        for (int u = 0; u < b.N; ++u) acc += dot3(sub3(vi, scale3(s, f3(dc[b.j[u]]))), b.J[u]);
+    });
     acc = group_sum<G>(acc);
-    if (T.valid && T.lane == 0 && D.div_out) D.div_out[D.pid[T.i]] = acc > 0.0f ? acc : 0.0f;
+    if (T.valid && T.lane == 0) D.div_out[D.pid[T.i]] = acc > 0.0f ? acc : 0.0f;
 }
 
 // ---- Weiler 2018 implicit viscosity (weiler18.py:21-401), slot order
@@ -1756,9 +1586,8 @@ __device__ __forceinline__ float visc_factor(const Dev& D, const SceneParams& P,
 // Setup (weiler18.py:381-396): 3x3 block-Jacobi inverse M_i^-1 of
 // I - dt mu_i/rho_i L_ii (weiler18.py:21-85), rhs = v - A v, r = rhs,
 // z = M^-1 r, dv = 0, p_prev = 0; partial r.z.
-template <int G>
-__device__ __forceinline__ double visc_setup_tile(const Dev& D, const SceneParams& P, const TileCtx& T) {
-    const int cnt = T.valid ? D.nbr_cnt[T.row] : 0;
+template <int G, class R>
+__device__ __forceinline__ double visc_setup_tile(R& rows, const Dev& D, const SceneParams& P, const TileCtx& T) {
     const bool fluid = T.valid && D.rflu[T.i] != 0.0f;
     float3 xi = make_float3(0.f, 0.f, 0.f), vi = xi;
     // vs holds every slot's {v, 1/rho if fluid} (written before the setup)
@@ -1771,13 +1600,10 @@ __device__ __forceinline__ double visc_setup_tile(const Dev& D, const SceneParam
 #pragma unroll
     for (int q = 0; q < 9; ++q) L[q] = 0.0f;
     float lx = 0.0f, ly = 0.0f, lz = 0.0f;
-    bool bad = false;
-    const int self = T.valid ? T.i : P.s_begin;
-    for (int k0 = 2 * T.lane; k0 < (fluid ? cnt : 0); k0 += G * PU) {
-        PairBatch b;
-        bad |= load_pairs<G>(D, T.row, xi, k0, cnt, self, P.s_begin, P.s_end, b);
+    rows.open(T.row, T.valid);
+    rows.each(T.row, xi, [&](const auto& b, int, size_t) {
 #pragma unroll
-        for (int u = 0; u < PU; ++u) {
+        for (int u = 0; u < b.N; ++u) {
             const int j = b.j[u];
             const float3 xij = sub3(xi, f3(__ldg(D.xm + j)));
             const float4 vj = D.vs[j];
@@ -1795,8 +1621,7 @@ __device__ __forceinline__ double visc_setup_tile(const Dev& D, const SceneParam
             ly += s * J.y;
             lz += s * J.z;
         }
-    }
-    if (bad) flag_bad(D, T.i, 5);
+    });
 #pragma unroll
     for (int q = 0; q < 9; ++q) L[q] = group_sum<G>(L[q]);
     lx = group_sum<G>(lx);
@@ -1845,15 +1670,14 @@ __device__ __forceinline__ double visc_setup_tile(const Dev& D, const SceneParam
 //   L(p_k) = L(z_k) + beta L(p_(k-1))
 // (exact for the linear L), so a neighbour contributes one 32-byte record
 // {z_j | 1/rho_j, x_j}; partial p.Ap.
-template <int G>
-__device__ __forceinline__ double visc_a_tile(const Dev& D, const SceneParams& P, const TileCtx& T, float beta,
+template <int G, class R>
+__device__ __forceinline__ double visc_a_tile(R& rows, const Dev& D, const SceneParams& P, const TileCtx& T, float beta,
                                               int it) {
     // {z | 1/rho, x}.  Only dynamic slots' records are ever written; a
     // static neighbour's record keeps the zeros of ivp_engine_create's
     // workspace clear, so its 1/rho = 0 removes it from the sum (the
     // reference's fluid-only `continue`) with finite arithmetic.
     const float4* cc = (it & 1) ? D.cg1 : D.cg0;
-    const int cnt = T.valid ? D.nbr_cnt[T.row] : 0;
     const bool fluid = T.valid && D.rflu[T.i] != 0.0f;
     float3 xi = make_float3(0.f, 0.f, 0.f), zi = xi;
     if (T.valid) {
@@ -1862,13 +1686,10 @@ __device__ __forceinline__ double visc_a_tile(const Dev& D, const SceneParams& P
     }
     const float eps2 = 0.01f * P.h * P.h;
     float lx = 0.0f, ly = 0.0f, lz = 0.0f;
-    bool bad = false;
-    const int self = T.valid ? T.i : P.s_begin;
-    for (int k0 = 2 * T.lane; k0 < (fluid ? cnt : 0); k0 += G * PU) {
-        PairBatch b;
-        bad |= load_pairs<G>(D, T.row, xi, k0, cnt, self, P.s_begin, P.s_end, b);
+    rows.open(T.row, T.valid);
+    rows.each(T.row, xi, [&](const auto& b, int, size_t) {
 #pragma unroll
-        for (int u = 0; u < PU; ++u) {
+        for (int u = 0; u < b.N; ++u) {
             float4 zj, xj;
             ld_rec(cc + 2 * b.j[u], zj, xj);
             const float3 xij = sub3(xi, f3(xj));
@@ -1878,8 +1699,7 @@ __device__ __forceinline__ double visc_a_tile(const Dev& D, const SceneParams& P
             ly += s * b.J[u].y;
             lz += s * b.J[u].z;
         }
-    }
-    if (bad) flag_bad(D, T.i, 6);
+    });
     lx = group_sum<G>(lx);
     ly = group_sum<G>(ly);
     lz = group_sum<G>(lz);
@@ -1993,9 +1813,8 @@ __global__ void k_slot_velocity(const Dev D) {
 // compute_divergence_jeske23 (jeske23.py:74-115): div_i = sum over fluid j of
 // m_j v_ij . grad W_ij = J_ij . v_ij.  Stores the slot's record for the
 // setup's neighbour gathers: {v, div} {rho, 1/rho if fluid}.
-template <int G>
-__device__ __forceinline__ void st_div_tile(const Dev& D, const SceneParams& P, const TileCtx& T) {
-    const int cnt = T.valid ? D.nbr_cnt[T.row] : 0;
+template <int G, class R>
+__device__ __forceinline__ void st_div_tile(R& rows, const Dev& D, const SceneParams& P, const TileCtx& T) {
     float3 xi = make_float3(0.f, 0.f, 0.f), vi = xi;
     float rfi = 0.0f;
     if (T.valid) {
@@ -2006,19 +1825,14 @@ __device__ __forceinline__ void st_div_tile(const Dev& D, const SceneParams& P, 
     }
     const bool fluid = T.valid && rfi != 0.0f;
     float acc = 0.0f;
-    bool bad = false;
-    const int self = T.valid ? T.i : P.s_begin;
-    for (int k0 = 2 * T.lane; k0 < (fluid ? cnt : 0); k0 += G * PU) {
-        PairBatch b;
-        bad |= load_pairs<G>(D, T.row, xi, k0, cnt, self, P.s_begin, P.s_end, b);
+    rows.open(T.row, T.valid);
+    rows.each(T.row, xi, [&](const auto& b, int, size_t) {
 #pragma unroll
-        for (int u = 0; u < PU; ++u) {
+        for (int u = 0; u < b.N; ++u) {
             const float4 vj = D.vs[b.j[u]];
-            const bool use = ((b.live >> u) & 1u) && vj.w != 0.0f;
-            acc += use ? dot3(sub3(vi, f3(vj)), b.J[u]) : 0.0f;
+            acc += vj.w != 0.0f ? dot3(sub3(vi, f3(vj)), b.J[u]) : 0.0f;
         }
-    }
-    if (bad) flag_bad(D, T.i, 7);
+    });
     acc = group_sum<G>(acc);
     if (T.valid && T.lane == 0) {
         D.st_rec[2 * T.i] = make_float4(vi.x, vi.y, vi.z, fluid ? acc : 0.0f);
@@ -2031,9 +1845,8 @@ __device__ __forceinline__ void st_div_tile(const Dev& D, const SceneParams& P, 
 // entry (the CG operator streams only that), the extra right-hand side b
 // (jeske23.py:190-237), the Jacobi inverse (jeske23.py:295-350),
 // rhs = v - M v + b, then r = rhs, z = M^-1 r, dv = 0, p_prev = 0; partial r.z.
-template <int G>
-__device__ __forceinline__ double st_setup_tile(const Dev& D, const SceneParams& P, const TileCtx& T) {
-    const int cnt = T.valid ? D.nbr_cnt[T.row] : 0;
+template <int G, class R>
+__device__ __forceinline__ double st_setup_tile(R& rows, const Dev& D, const SceneParams& P, const TileCtx& T) {
     float3 xi = make_float3(0.f, 0.f, 0.f), vi = xi;
     float mi = 1.0f, rhoi = 1.0f, divi = 0.0f, rfi = 0.0f;
     if (T.valid) {
@@ -2050,20 +1863,17 @@ __device__ __forceinline__ double st_setup_tile(const Dev& D, const SceneParams&
     const bool fluid = T.valid && rfi != 0.0f;
     const float d = P.st_d, hs = P.st_h, dt = P.dt;
     float bx = 0.f, by = 0.f, bz = 0.f, sx = 0.f, sy = 0.f, sz = 0.f, ds = 0.f;
-    bool bad = false;
-    const int self = T.valid ? T.i : P.s_begin;
-    float2* wrow = D.st_w + (size_t)T.row * D.stride;
-    for (int k0 = 2 * T.lane; k0 < (fluid ? cnt : 0); k0 += G * PU) {
-        PairBatch b;
-        bad |= load_pairs<G>(D, T.row, xi, k0, cnt, self, P.s_begin, P.s_end, b);
+    rows.open(T.row, T.valid);
+    rows.each(T.row, xi, [&](const auto& b, int k0, size_t e) {
+        float wj[b.N];
 #pragma unroll
-        for (int u = 0; u < PU; ++u) {
+        for (int u = 0; u < b.N; ++u) {
             const int k = k0 + (u >> 1) * 2 * G + (u & 1);
             const int j = b.j[u];
             const float4 xj4 = __ldg(D.xm + j);
             float4 q0, q1;
             ld_rec(D.st_rec + 2 * j, q0, q1);
-            const bool use = ((b.live >> u) & 1u) && q1.y != 0.0f;
+            const bool use = fluid && k < rows.cnt && q1.y != 0.0f;
             const float3 xij = sub3(xi, f3(xj4));
             const float r = sqrtf(norm2_rn(xij));
             float gt = 0.0f;
@@ -2080,7 +1890,7 @@ __device__ __forceinline__ double st_setup_tile(const Dev& D, const SceneParams&
             }
             const float mbar = 0.5f * (mi + xj4.w);
             const float w = mbar * gt;
-            if (k < cnt) wrow[k] = make_float2(__int_as_float(j), use ? w : 0.0f);
+            wj[u] = use ? w : 0.0f;
             if (use) {
                 ds += w;
                 if (gt != 0.0f) {
@@ -2093,8 +1903,11 @@ __device__ __forceinline__ double st_setup_tile(const Dev& D, const SceneParams&
                 }
             }
         }
-    }
-    if (bad) flag_bad(D, T.i, 8);
+#pragma unroll
+        for (int u = 0; u < b.N; u += 2)
+            *reinterpret_cast<float4*>(D.st_w + e + lane_entry(u)) =
+                make_float4(__int_as_float(b.j[u]), wj[u], __int_as_float(b.j[u + 1]), wj[u + 1]);
+    });
     bx = group_sum<G>(bx);
     by = group_sum<G>(by);
     bz = group_sum<G>(bz);
@@ -2148,35 +1961,25 @@ __device__ __forceinline__ double st_a_tile(const Dev& D, const SceneParams& P, 
     }
     float sx = 0.f, sy = 0.f, sz = 0.f;
     const int self = T.valid ? T.i : P.s_begin;
-    // list entries k, k+1 as one 16-byte load {j, w, j, w} (rows start on
-    // 512-byte boundaries and k is even)
-    const float4* wrow = reinterpret_cast<const float4*>(D.st_w + (size_t)T.row * D.stride);
-    for (int k0 = 2 * T.lane; k0 < (fluid ? cnt : 0); k0 += G * PU) {
-        int jj[PU];
-        float ww[PU];
-#pragma unroll
-        for (int u = 0; u < PU / 2; ++u) {
-            const int k = k0 + u * 2 * G;
-            float4 e = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (k < cnt) e = wrow[k >> 1];
-            const bool in0 = k < cnt, in1 = k + 1 < cnt;
-            jj[2 * u] = in0 ? __float_as_int(e.x) : self;
-            ww[2 * u] = in0 ? e.y : 0.0f;
-            jj[2 * u + 1] = in1 ? __float_as_int(e.z) : self;
-            ww[2 * u + 1] = in1 ? e.w : 0.0f;
-        }
-#pragma unroll
-        for (int u = 0; u < PU; ++u) {
-            const int j = (jj[u] >= P.s_begin && jj[u] < P.s_end) ? jj[u] : self;
-            const float3 zj = f3(ld_vec(D.stz + j));
-            const float w = ww[u];
-            if (w != 0.0f) {
-                sx += w * (zi.x - zj.x);
-                sy += w * (zi.y - zj.y);
-                sz += w * (zi.z - zj.z);
-            }
-        }
+    // the entries where `each` reads the rows', {j, w} of a pair in 16 bytes
+    const int lane = threadIdx.x & 31;
+    const float4* q = reinterpret_cast<const float4*>(D.st_w + (size_t)(T.row - lane / G) * D.stride) + lane;
+    auto add = [&](const float4& e) {
+        const float3 za = f3(ld_vec(D.stz + __float_as_int(e.x))), zb = f3(ld_vec(D.stz + __float_as_int(e.z)));
+        sx += e.y * (zi.x - za.x);
+        sy += e.y * (zi.y - za.y);
+        sz += e.y * (zi.z - za.z);
+        sx += e.w * (zi.x - zb.x);
+        sy += e.w * (zi.y - zb.y);
+        sz += e.w * (zi.z - zb.z);
+    };
+    int k = 0;
+    for (; k + 2 * G < cnt; k += 4 * G, q += 64) {
+        const float4 e01 = q[0], e23 = q[32];
+        add(e01);
+        add(e23);
     }
+    if (k < cnt) add(q[0]);
     sx = group_sum<G>(sx);
     sy = group_sum<G>(sy);
     sz = group_sum<G>(sz);
@@ -2239,9 +2042,8 @@ __device__ __forceinline__ void st_b_tile(const Dev& D, const TileCtx& T, float 
 
 // pj_head_fused (prj.py:17-55): dt_v = dt_v_0 - dt^2 J^T lambda / max(m, 1e-6),
 // J^T lambda in gather form (m_j l_i + m_i l_j) grad W = (l_i + m_i q_j) J_ij.
-template <int G>
-__device__ __forceinline__ void pj_head_tile(const Dev& D, const SceneParams& P, const TileCtx& T) {
-    const int cnt = T.valid ? D.nbr_cnt[T.row] : 0;
+template <int G, class R>
+__device__ __forceinline__ void pj_head_tile(R& rows, const Dev& D, const SceneParams& P, const TileCtx& T) {
     float3 xi = make_float3(0.f, 0.f, 0.f);
     float li = 0.0f, mi = 1.0f;
     if (T.valid) {
@@ -2251,17 +2053,16 @@ __device__ __forceinline__ void pj_head_tile(const Dev& D, const SceneParams& P,
         li = D.fk[T.i];
     }
     float ax = 0.0f, ay = 0.0f, az = 0.0f;
-    const int self = T.valid ? T.i : P.s_begin;
-    const bool bad = pair_loop<G>(D, T.row, xi, cnt, T.lane, self, P.s_begin, P.s_end, [&](const PairBatch& b) {
+    rows.open(T.row, T.valid);
+    rows.each(T.row, xi, [&](const auto& b, int, size_t) {
 #pragma unroll
-        for (int u = 0; u < PU; ++u) {
+        for (int u = 0; u < b.N; ++u) {
             const float wgt = li + mi * D.q[b.j[u]];
             ax += wgt * b.J[u].x;
             ay += wgt * b.J[u].y;
             az += wgt * b.J[u].z;
         }
     });
-    if (bad) flag_bad(D, T.i, 11);
     ax = group_sum<G>(ax);
     ay = group_sum<G>(ay);
     az = group_sum<G>(az);
@@ -2274,24 +2075,23 @@ __device__ __forceinline__ void pj_head_tile(const Dev& D, const SceneParams& P,
 
 // pj_tail_fused (prj.py:58-117): r = dt J dt_v + c, lambda = max(lambda +
 // omega r D^-1, 0); partial max(r / max(rho0, 1e-6), 0).
-template <int G>
-__device__ __forceinline__ double pj_tail_tile(const Dev& D, const SceneParams& P, const TileCtx& T) {
-    const int cnt = T.valid ? D.nbr_cnt[T.row] : 0;
+template <int G, class R>
+__device__ __forceinline__ double pj_tail_tile(R& rows, const Dev& D, const SceneParams& P, const TileCtx& T) {
     float3 xi = make_float3(0.f, 0.f, 0.f), vi = xi;
     if (T.valid) {
         xi = f3(D.xm[T.i]);
         vi = f3(D.d0[T.i]);
     }
     float acc = 0.0f;
-    const int self = T.valid ? T.i : P.s_begin;
-    const bool bad = pair_loop<G>(D, T.row, xi, cnt, T.lane, self, P.s_begin, P.s_end, [&](const PairBatch& b) {
+    rows.open(T.row, T.valid);
+    rows.each(T.row, xi, [&](const auto& b, int, size_t) {
 #pragma unroll
-        for (int u = 0; u < PU; ++u) acc += dot3(sub3(vi, f3(D.d0[b.j[u]])), b.J[u]);
+        for (int u = 0; u < b.N; ++u) acc += dot3(sub3(vi, f3(D.d0[b.j[u]])), b.J[u]);
     });
-    if (bad) flag_bad(D, T.i, 12);
     acc = group_sum<G>(acc);
     double part = 0.0;
     if (T.valid && T.lane == 0) {
+        if (D.div_out) D.jd[T.i] = acc;
         const float r = acc + D.c[T.i];
         const float l = D.fk[T.i] + P.omega * r * D.kd[T.i];
         const float lc = l > 0.0f ? l : 0.0f;
@@ -2353,18 +2153,20 @@ __global__ void k_prj_begin(const Dev D) {
 template <int G, int BLOCK>
 __global__ void __launch_bounds__(BLOCK) k_pj_head(const Dev D) {
     const TileCtx T = tile_ctx<G>(D, blockIdx.x);
-    if (D.ctl[T.sc].outer_active) pj_head_tile<G>(D, D.scenes[T.sc], T);
+    Rows<G, READ_ANY> rows(D);
+    if (D.ctl[T.sc].outer_active) pj_head_tile<G>(rows, D, D.scenes[T.sc], T);
 }
 
 template <int G, int BLOCK>
 __global__ void __launch_bounds__(BLOCK) k_pj_tail(const Dev D) {
     const TileCtx T = tile_ctx<G>(D, blockIdx.x);
+    Rows<G, READ_ANY> rows(D);
     __shared__ int sh_active;
     if (threadIdx.x == 0) sh_active = D.ctl[T.sc].outer_active;
     __syncthreads();
     const bool active = sh_active != 0;
     double part = 0.0;
-    if (active) part = pj_tail_tile<G>(D, D.scenes[T.sc], T);
+    if (active) part = pj_tail_tile<G>(rows, D, D.scenes[T.sc], T);
     block_finish<BLOCK>(D, T.sc, active, part, K_PJ_TAIL);
 }
 
@@ -2383,6 +2185,7 @@ __global__ void k_prj_end(const Dev D) {
 template <int G, int BLOCK>
 __global__ void __launch_bounds__(BLOCK) k_pack(const Dev D) {
     const TileCtx T = tile_ctx<G>(D, blockIdx.x);
+    Rows<G, READ_ANY> rows(D);
     __shared__ int sh_active, sh_it;
     if (threadIdx.x == 0) {
         sh_active = D.ctl[T.sc].outer_active;
@@ -2391,13 +2194,14 @@ __global__ void __launch_bounds__(BLOCK) k_pack(const Dev D) {
     __syncthreads();
     const bool active = sh_active != 0;
     double part = 0.0;
-    if (active) part = pack_tile<G>(D, D.scenes[T.sc], T, sh_it);
+    if (active) part = pack_tile<G>(rows, D, D.scenes[T.sc], T, sh_it);
     block_finish<BLOCK>(D, T.sc, active, part, K_PACK);
 }
 
 template <int G, int BLOCK>
 __global__ void __launch_bounds__(BLOCK) k_rhs(const Dev D) {
     const TileCtx T = tile_ctx<G>(D, blockIdx.x);
+    Rows<G, READ_ANY> rows(D);
     __shared__ int sh_active;
     __shared__ int sh_outer;
     if (threadIdx.x == 0) {
@@ -2407,13 +2211,14 @@ __global__ void __launch_bounds__(BLOCK) k_rhs(const Dev D) {
     __syncthreads();
     const bool active = sh_active != 0;
     double part = 0.0;
-    if (active) part = rhs_tile<G>(D, D.scenes[T.sc], T, (sh_outer & 1) ? D.d1 : D.d0);
+    if (active) part = rhs_tile<G>(rows, D, D.scenes[T.sc], T, (sh_outer & 1) ? D.d1 : D.d0);
     block_finish<BLOCK>(D, T.sc, active, part, K_RHS);
 }
 
 template <int G, int BLOCK>
 __global__ void __launch_bounds__(BLOCK) k_cg_a(const Dev D) {
     const TileCtx T = tile_ctx<G>(D, blockIdx.x);
+    Rows<G, READ_ANY> rows(D);
     __shared__ int sh_active, sh_it;
     __shared__ float sh_beta;
     if (threadIdx.x == 0) {
@@ -2425,13 +2230,14 @@ __global__ void __launch_bounds__(BLOCK) k_cg_a(const Dev D) {
     __syncthreads();
     const bool active = sh_active != 0;
     double part = 0.0;
-    if (active) part = cga_tile<G>(D, D.scenes[T.sc], T, sh_beta, sh_it);
+    if (active) part = cga_tile<G>(rows, D, D.scenes[T.sc], T, sh_beta, sh_it);
     block_finish<BLOCK>(D, T.sc, active, part, K_CG_A);
 }
 
 template <int G, int BLOCK>
 __global__ void __launch_bounds__(BLOCK) k_cg_b(const Dev D) {
     const TileCtx T = tile_ctx<G>(D, blockIdx.x);
+    Rows<G, READ_ANY> rows(D);
     __shared__ int sh_active, sh_it, sh_outer;
     __shared__ float sh_alpha;
     if (threadIdx.x == 0) {
@@ -2444,15 +2250,16 @@ __global__ void __launch_bounds__(BLOCK) k_cg_b(const Dev D) {
     __syncthreads();
     const bool active = sh_active != 0;
     double part = 0.0;
-    if (active) part = cgb_tile<G>(D, D.scenes[T.sc], T, sh_alpha, sh_it, (sh_outer & 1) ? D.d1 : D.d0);
+    if (active) part = cgb_tile<G>(rows, D, D.scenes[T.sc], T, sh_alpha, sh_it, (sh_outer & 1) ? D.d1 : D.d0);
     block_finish<BLOCK>(D, T.sc, active, part, K_CG_B);
 }
 
 template <int G, int BLOCK>
 __global__ void __launch_bounds__(BLOCK) k_divergence(const Dev D) {
     const TileCtx T = tile_ctx<G>(D, blockIdx.x);
+    Rows<G, READ_ANY> rows(D);
     const SceneParams& P = D.scenes[T.sc];
-    div_tile<G>(D, P, T, P.solver == SOLVER_PRJ ? 0 : D.ctl[T.sc].outer_it);
+    div_tile<G>(rows, D, P, T, D.ctl[T.sc]);
 }
 
 // viscosity, one launch per phase
@@ -2470,25 +2277,28 @@ __global__ void k_visc_begin(const Dev D) {
 template <int G, int BLOCK>
 __global__ void __launch_bounds__(BLOCK) k_st_div(const Dev D) {
     const TileCtx T = tile_ctx<G>(D, blockIdx.x);
-    if (D.ctl[T.sc].v_on) st_div_tile<G>(D, D.scenes[T.sc], T);
+    Rows<G, READ_ANY> rows(D);
+    if (D.ctl[T.sc].v_on) st_div_tile<G>(rows, D, D.scenes[T.sc], T);
 }
 
 template <int G, int BLOCK>
 __global__ void __launch_bounds__(BLOCK) k_visc_setup(const Dev D) {
     const TileCtx T = tile_ctx<G>(D, blockIdx.x);
+    Rows<G, READ_ANY> rows(D);
     __shared__ int sh_active;
     if (threadIdx.x == 0) sh_active = D.ctl[T.sc].v_on;
     __syncthreads();
     const bool active = sh_active != 0;
     double part = 0.0;
     if (active)
-        part = D.force == FORCE_ST ? st_setup_tile<G>(D, D.scenes[T.sc], T) : visc_setup_tile<G>(D, D.scenes[T.sc], T);
+        part = D.force == FORCE_ST ? st_setup_tile<G>(rows, D, D.scenes[T.sc], T) : visc_setup_tile<G>(rows, D, D.scenes[T.sc], T);
     block_finish<BLOCK>(D, T.sc, active, part, K_V_SETUP);
 }
 
 template <int G, int BLOCK>
 __global__ void __launch_bounds__(BLOCK) k_visc_a(const Dev D) {
     const TileCtx T = tile_ctx<G>(D, blockIdx.x);
+    Rows<G, READ_ANY> rows(D);
     __shared__ int sh_active, sh_it;
     __shared__ float sh_beta;
     if (threadIdx.x == 0) {
@@ -2502,7 +2312,7 @@ __global__ void __launch_bounds__(BLOCK) k_visc_a(const Dev D) {
     double part = 0.0;
     if (active)
         part = D.force == FORCE_ST ? st_a_tile<G>(D, D.scenes[T.sc], T, sh_beta, sh_it)
-                                   : visc_a_tile<G>(D, D.scenes[T.sc], T, sh_beta, sh_it);
+                                   : visc_a_tile<G>(rows, D, D.scenes[T.sc], T, sh_beta, sh_it);
     block_finish<BLOCK>(D, T.sc, active, part, K_V_A);
 }
 
@@ -2583,27 +2393,46 @@ __device__ __forceinline__ SceneCtl ctl_load(const SceneCtl* p) {
 // Scenes up to this count are summed one after another by the whole CTA;
 // more are spread over the warps, one scene per warp.
 constexpr int kBlockSumScenes = 2;
+// Scenes up to this count have their parameters in shared memory.
+constexpr int kParamScenes = 4;
 
 // Scene sums of a phase's tile partials (`partial`, second partial at
 // `partial + n_tiles`) into sum_sh / sum_sh2, then every active scene's
 // decision on the CTA's control-block copies.  `publish`: this CTA writes the
-// decided blocks (and the history) to global memory.
+// history, and, where the other CTAs wait for its decisions, the decided
+// blocks to global memory (else they are published at the end of the solve).
 template <int BLOCK>
 __device__ void reduce_and_decide(const Dev& D, int kind, const double* partial, double* sum_sh, double* sum_sh2,
-                                  SceneCtl* sc_sh, double* red_sh, bool publish) {
+                                  SceneCtl* sc_sh, double* red_sh, bool publish, const SceneParams* params) {
     const int ns = D.n_scenes;
     if (ns <= kBlockSumScenes) {
+        // scene_sum_block's association with two CTA barriers per scene: four
+        // warps add the lanes, the first warp walks the tree and decides
+        const int t = threadIdx.x;
         for (int s = 0; s < ns; ++s) {
-            if (!phase_active(sc_sh[s], kind)) continue;
-            const SceneParams& P = D.scenes[s];
-            const double v = scene_sum_block<BLOCK>(partial, P.tile_begin, P.tile_end, red_sh);
-            const double v2 =
-                kind == K_V_B ? scene_sum_block<BLOCK>(partial + D.n_tiles, P.tile_begin, P.tile_end, red_sh) : 0.0;
-            if (threadIdx.x == 0) {
-                sum_sh[s] = v;
-                sum_sh2[s] = v2;
+            if (!phase_active(sc_sh[s], kind)) continue;  // the same in every thread
+            const SceneParams& P = params[s];
+            if (t < 128) {
+                red_sh[t] = lane_sum128(partial, P.tile_begin + t, P.tile_end);
+                if (kind == K_V_B) red_sh[128 + t] = lane_sum128(partial + D.n_tiles, P.tile_begin + t, P.tile_end);
             }
+            __syncthreads();
+            if (t < 32) {
+                const double v = tree32((red_sh[t] + red_sh[t + 64]) + (red_sh[t + 32] + red_sh[t + 96]));
+                double v2 = 0.0;
+                if (kind == K_V_B)
+                    v2 = tree32((red_sh[t + 128] + red_sh[t + 192]) + (red_sh[t + 160] + red_sh[t + 224]));
+                if (t == 0) {
+                    scene_decide(D, P, sc_sh[s], kind, v, publish, v2);
+                    if (publish && !D.bar_all_reduce) {
+                        D.ctl[s] = sc_sh[s];
+                        __threadfence();
+                    }
+                }
+            }
+            __syncthreads();
         }
+        return;
     } else {
         const int warp = threadIdx.x >> 5;
         for (int s = warp; s < ns; s += BLOCK / 32) {
@@ -2621,7 +2450,7 @@ __device__ void reduce_and_decide(const Dev& D, int kind, const double* partial,
     for (int s = threadIdx.x; s < ns; s += BLOCK) {
         SceneCtl& c = sc_sh[s];
         if (!phase_active(c, kind)) continue;
-        scene_decide(D, D.scenes[s], c, kind, sum_sh[s], publish, sum_sh2[s]);
+        scene_decide(D, params[s], c, kind, sum_sh[s], publish, sum_sh2[s]);
         if (publish) {
             D.ctl[s] = c;
             __threadfence();
@@ -2633,18 +2462,18 @@ __device__ void reduce_and_decide(const Dev& D, int kind, const double* partial,
 // Barrier in which every CTA reduces: after all CTAs arrived (one monotonic
 // arrival counter, `target` = this barrier's count), each CTA sums the
 // partials and runs the decisions itself -- same inputs, same code, same
-// bits -- so no control block has to travel back.  CTA 0 publishes them.
+// bits -- so no control block has to travel back.  CTA 0 writes the history.
 // Used when the partials are few (one or two scenes); the partials alternate
 // between two buffers by barrier parity, so a CTA that runs ahead into the
 // next phase never overwrites partials another CTA is still reading.
 template <int BLOCK>
 __device__ bool grid_all_reduce_barrier(const Dev& D, int kind, const double* partial, int* sh_flag,
                                         double* sum_sh, double* sum_sh2, SceneCtl* sc_sh, double* red_sh,
-                                        unsigned target) {
+                                        unsigned target, const SceneParams* params) {
     __syncthreads();
     if (threadIdx.x == 0) {
-        __threadfence();
-        atomicAdd(D.bar_count, 1u);
+        // releases the whole CTA's writes (ordered before it by the barrier)
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(D.bar_count) : "memory");
         volatile unsigned* cnt = D.bar_count;
         int ok = 1;
         const unsigned long long t0 = globaltimer_ns();
@@ -2661,13 +2490,13 @@ __device__ bool grid_all_reduce_barrier(const Dev& D, int kind, const double* pa
     }
     __syncthreads();
     if (!sh_flag[1]) return false;
-    if (kind >= 0) reduce_and_decide<BLOCK>(D, kind, partial, sum_sh, sum_sh2, sc_sh, red_sh, blockIdx.x == 0);
+    if (kind >= 0) reduce_and_decide<BLOCK>(D, kind, partial, sum_sh, sum_sh2, sc_sh, red_sh, blockIdx.x == 0, params);
     return true;
 }
 
 template <int BLOCK>
 __device__ bool grid_reduce_barrier(const Dev& D, int kind, const double* partial, int* sh_flag, double* sum_sh,
-                                    double* sum_sh2, SceneCtl* sc_sh, double* red_sh) {
+                                    double* sum_sh2, SceneCtl* sc_sh, double* red_sh, const SceneParams* params) {
     unsigned g = 0;
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -2679,7 +2508,7 @@ __device__ bool grid_reduce_barrier(const Dev& D, int kind, const double* partia
     __syncthreads();
     if (sh_flag[0]) {
         __threadfence();
-        if (kind >= 0) reduce_and_decide<BLOCK>(D, kind, partial, sum_sh, sum_sh2, sc_sh, red_sh, true);
+        if (kind >= 0) reduce_and_decide<BLOCK>(D, kind, partial, sum_sh, sum_sh2, sc_sh, red_sh, true, params);
         __syncthreads();
         if (threadIdx.x == 0) {
             *D.bar_count = 0;
@@ -2711,32 +2540,59 @@ constexpr int kFlushTiles = 16;
 // Phase driver shared by the persistent kernels: tiles dealt round-robin over
 // the CTAs, local copies of the control blocks, one grid barrier + reduction
 // per phase.
-template <int G, int BLOCK>
+template <int BLOCK>
+struct PhaseShared {
+    double red[256];
+    double warp_sum[2][kFlushTiles][BLOCK / 32];  // parked per-warp sums of the CTA's tiles
+    int tile[kFlushTiles];
+    int flag[2], any;
+};
+
+template <int G, int BLOCK, int F>
 struct Phaser {
     const Dev& D;
+    PhaseShared<BLOCK>& S;
     double* sum_sh;
     double* sum_sh2;
     SceneCtl* sc_sh;
-    double* red_sh;
-    int* flag_sh;
-    int* any_sh;
     long long phases;
 
     int* act_sh;   // [n_scenes + 1] exclusive prefix of the phase's active tile counts
     int* tb_sh;    // [n_scenes] first tile of each scene
     int* tn_sh;    // [n_scenes] tile count of each scene
+    const SceneParams* pp;  // the scenes' parameters (shared memory where they are few)
 
-    __device__ Phaser(const Dev& d, double* dyn, double* red, int* flag, int* anyp)
-        : D(d), red_sh(red), flag_sh(flag), any_sh(anyp), phases(0) {
-        sum_sh = dyn;
-        sum_sh2 = dyn + D.n_scenes;
-        sc_sh = reinterpret_cast<SceneCtl*>(dyn + 2 * D.n_scenes);
+    // dynamic shared memory: control blocks, tile tables, a few scenes' parameters
+    static __host__ __device__ size_t shared_bytes(int n_scenes) {
+        return (size_t)n_scenes * (2 * sizeof(double) + sizeof(SceneCtl) + 3 * sizeof(int)) + sizeof(int) +
+                         (n_scenes <= kParamScenes ? n_scenes * sizeof(SceneParams) + sizeof(double) : 0);
+    }
+
+    __device__ Phaser(const Dev& d, unsigned char* dyn, PhaseShared<BLOCK>& sh) : D(d), S(sh), phases(0) {
+        sum_sh = reinterpret_cast<double*>(dyn);
+        sum_sh2 = sum_sh + D.n_scenes;
+        sc_sh = reinterpret_cast<SceneCtl*>(sum_sh + 2 * D.n_scenes);
         act_sh = reinterpret_cast<int*>(sc_sh + D.n_scenes);
         tb_sh = act_sh + D.n_scenes + 1;
         tn_sh = tb_sh + D.n_scenes;
+        pp = D.scenes;
+        if (D.n_scenes <= kParamScenes) {
+            // a few scenes' parameters in shared memory: a phase would read
+            // them from L2 again after every grid barrier
+            int* q = tn_sh + D.n_scenes;
+            q += ((reinterpret_cast<uintptr_t>(q) & 7) != 0);
+            const int* from = reinterpret_cast<const int*>(D.scenes);
+            for (int k = threadIdx.x; k < (int)(D.n_scenes * sizeof(SceneParams) / sizeof(int)); k += BLOCK) q[k] = from[k];
+            pp = reinterpret_cast<const SceneParams*>(q);
+        }
         for (int s = threadIdx.x; s < D.n_scenes; s += BLOCK) {
             tb_sh[s] = D.scenes[s].tile_begin;
             tn_sh[s] = D.scenes[s].tile_end - D.scenes[s].tile_begin;
+            act_sh[s] = 0;
+        }
+        if (threadIdx.x == 0) {
+            // one scene: every phase that runs has all of its tiles
+            act_sh[D.n_scenes] = D.n_scenes == 1 ? D.scenes[0].tile_end - D.scenes[0].tile_begin : 0;
         }
         __syncthreads();
     }
@@ -2775,6 +2631,8 @@ struct Phaser {
         return lo;
     }
 
+    Rows<G, F> rows{D};
+
     unsigned nbar = 0;  // barriers passed by this launch (the same count in every CTA)
 
     // this phase's partial buffer (two per tile, alternating by barrier parity)
@@ -2784,9 +2642,9 @@ struct Phaser {
         const double* part = partials();
         ++nbar;
         if (D.bar_all_reduce)
-            return grid_all_reduce_barrier<BLOCK>(D, kind, part, flag_sh, sum_sh, sum_sh2, sc_sh, red_sh,
-                                                  nbar * gridDim.x);
-        return grid_reduce_barrier<BLOCK>(D, kind, part, flag_sh, sum_sh, sum_sh2, sc_sh, red_sh);
+            return grid_all_reduce_barrier<BLOCK>(D, kind, part, S.flag, sum_sh, sum_sh2, sc_sh, S.red,
+                                                  nbar * gridDim.x, pp);
+        return grid_reduce_barrier<BLOCK>(D, kind, part, S.flag, sum_sh, sum_sh2, sc_sh, S.red, pp);
     }
 
     __device__ void refresh() {
@@ -2795,28 +2653,31 @@ struct Phaser {
     }
 
     __device__ bool any(int kind) {
+        if (D.n_scenes <= kBlockSumScenes) {
+            // every thread looks (the control blocks were synchronised)
+            bool a = false;
+            for (int s = 0; s < D.n_scenes; ++s) a |= phase_active(sc_sh[s], kind);
+            return a;
+        }
         if (threadIdx.x == 0) {
             int a = 0;
             for (int s = 0; s < D.n_scenes; ++s) a |= phase_active(sc_sh[s], kind) ? 1 : 0;
-            *any_sh = a;
+            S.any = a;
         }
         __syncthreads();
-        const bool r = *any_sh != 0;
+        const bool r = S.any != 0;
         __syncthreads();
         return r;
     }
 
-    // VISC selects the phase family compiled into this kernel (each
-    // persistent kernel keeps its own register budget)
-    // The phase's active tiles (those of the scenes active in `kind`) are
+    // One phase: the active tiles (those of the scenes active in KIND) are
     // split evenly over the grid, so scenes that converged early leave no CTA
-    // idle while others work through a converging scene's tiles.
-    // MODE selects the phase family compiled into the kernel: MODE_IP, or a
-    // non-pressure force (FORCE_VISC / FORCE_ST as MODE_FORCE + force); each
-    // persistent kernel keeps its own register budget
-    template <int MODE>
-    __device__ bool run(int kind) {
-        active_prefix(kind);
+    // idle while others work through a converging scene's tiles.  Each phase
+    // is compiled on its own, so that its registers are its tile body's alone.
+    template <int KIND, int FORCE = FORCE_VISC>
+    __device__ bool run() {
+        constexpr int kind = KIND;
+        if (D.n_scenes > 1) active_prefix(kind);
         const int A = act_sh[D.n_scenes];
         // active tiles dealt round-robin: at any moment the CTAs work on one
         // window of consecutive tiles, whose rows and neighbour records are
@@ -2828,8 +2689,8 @@ struct Phaser {
         // block_sum_d does.  Warps run ahead into the next tile instead of
         // waiting for a CTA-wide reduction after every tile.
         constexpr int NW = BLOCK / 32;
-        __shared__ double ws_sh[2][kFlushTiles][NW];
-        __shared__ int wt_sh[kFlushTiles];
+        auto& ws_sh = S.warp_sum;
+        auto& wt_sh = S.tile;
         const int wid = threadIdx.x >> 5, wl = threadIdx.x & 31;
         int nb = 0;
         auto flush = [&]() {
@@ -2845,8 +2706,7 @@ struct Phaser {
                 }
                 if (wl == 0) {
                     pb[wt_sh[s]] = t1;
-                    pb[D.n_tiles + wt_sh[s]] = t2;
-                    __threadfence();
+                    if (kind == K_V_B) pb[D.n_tiles + wt_sh[s]] = t2;
                 }
             }
             __syncthreads();
@@ -2856,7 +2716,7 @@ struct Phaser {
         for (int a = blockIdx.x; a < A; a += gridDim.x) {
             while (a >= act_sh[sc + 1]) ++sc;
             const int t = tb_sh[sc] + (a - act_sh[sc]);
-            const SceneParams& P = D.scenes[sc];
+            const SceneParams& P = pp[sc];
             TileCtx T;
             {
                 // the context computed from the scene's layout instead of
@@ -2876,29 +2736,30 @@ struct Phaser {
             }
             const SceneCtl& C = sc_sh[T.sc];
             double part = 0.0, part2 = 0.0;
-            if constexpr (MODE == MODE_FORCE + FORCE_ST) {
-                if (kind == K_ST_DIV) {
-                    st_div_tile<G>(D, P, T);
-                    continue;  // no reduction
-                }
-                if (kind == K_V_SETUP) part = st_setup_tile<G>(D, P, T);
-                else if (kind == K_V_A) part = st_a_tile<G>(D, P, T, (float)C.v_beta, C.v_it);
-                else st_b_tile<G>(D, T, (float)C.v_alpha, C.v_it, &part, &part2);
-            } else if constexpr (MODE == MODE_PRJ) {
-                if (kind == K_PJ_HEAD) {
-                    pj_head_tile<G>(D, P, T);
-                    continue;  // no reduction
-                }
-                part = pj_tail_tile<G>(D, P, T);
-            } else if constexpr (MODE == MODE_FORCE + FORCE_VISC) {
-                if (kind == K_V_SETUP) part = visc_setup_tile<G>(D, P, T);
-                else if (kind == K_V_A) part = visc_a_tile<G>(D, P, T, (float)C.v_beta, C.v_it);
+            if constexpr (KIND == K_ST_DIV) {
+                st_div_tile<G>(rows, D, P, T);
+                continue;  // no reduction
+            } else if constexpr (KIND == K_PJ_HEAD) {
+                pj_head_tile<G>(rows, D, P, T);
+                continue;  // no reduction
+            } else if constexpr (KIND == K_PJ_TAIL) {
+                part = pj_tail_tile<G>(rows, D, P, T);
+            } else if constexpr (KIND == K_V_SETUP) {
+                part = FORCE == FORCE_ST ? st_setup_tile<G>(rows, D, P, T) : visc_setup_tile<G>(rows, D, P, T);
+            } else if constexpr (KIND == K_V_A) {
+                part = FORCE == FORCE_ST ? st_a_tile<G>(D, P, T, (float)C.v_beta, C.v_it)
+                                         : visc_a_tile<G>(rows, D, P, T, (float)C.v_beta, C.v_it);
+            } else if constexpr (KIND == K_V_B) {
+                if constexpr (FORCE == FORCE_ST) st_b_tile<G>(D, T, (float)C.v_alpha, C.v_it, &part, &part2);
                 else visc_b_tile<G>(D, T, (float)C.v_alpha, C.v_it, &part, &part2);
+            } else if constexpr (KIND == K_PACK) {
+                part = pack_tile<G>(rows, D, P, T, C.outer_it);
+            } else if constexpr (KIND == K_RHS) {
+                part = rhs_tile<G>(rows, D, P, T, (C.outer_it & 1) ? D.d1 : D.d0);
+            } else if constexpr (KIND == K_CG_A) {
+                part = cga_tile<G>(rows, D, P, T, (float)C.beta, C.cg_it);
             } else {
-                if (kind == K_PACK) part = pack_tile<G>(D, P, T, C.outer_it);
-                else if (kind == K_RHS) part = rhs_tile<G>(D, P, T, (C.outer_it & 1) ? D.d1 : D.d0);
-                else if (kind == K_CG_A) part = cga_tile<G>(D, P, T, (float)C.beta, C.cg_it);
-                else part = cgb_tile<G>(D, P, T, (float)C.alpha, C.cg_it, (C.outer_it & 1) ? D.d1 : D.d0);
+                part = cgb_tile<G>(rows, D, P, T, (float)C.alpha, C.cg_it, (C.outer_it & 1) ? D.d1 : D.d0);
             }
             const double w1 = warp_sum_d(part);
             const double w2 = kind == K_V_B ? warp_sum_d(part2) : 0.0;
@@ -2916,12 +2777,12 @@ struct Phaser {
             // a barrier publishes it
             if (blockIdx.x == 0 && threadIdx.x == 0) {
                 for (int s = 0; s < D.n_scenes; ++s) {
-                    SceneCtl c = ctl_load(D.ctl + s);
+                    SceneCtl c = sc_sh[s];
                     if (c.outer_active || c.solve_pending || c.cg_active || c.v_active) {
                         c.status = IVP_TIMEOUT_;
                         c.outer_active = c.solve_pending = c.cg_active = c.v_active = 0;
-                        D.ctl[s] = c;
                     }
+                    D.ctl[s] = c;
                 }
                 D.flags->timeout = 1;
             }
@@ -2947,13 +2808,11 @@ constexpr int persist_min_blocks() { return IVP_PERSIST_THREADS / BLOCK > 0 ? IV
 // One implicit non-pressure solve of every scene that enables it, in one
 // persistent cooperative launch: Weiler 2018 viscosity (weiler18.py:371-401)
 // or Jeske 2023 surface tension (jeske23.py:585-655); D.force == FORCE.
-template <int G, int BLOCK, int FORCE>
+template <int G, int BLOCK, int F, int FORCE>
 __global__ void __launch_bounds__(BLOCK, persist_min_blocks<BLOCK>()) k_force_persistent(const Dev D) {
-    constexpr int M = MODE_FORCE + FORCE;
-    extern __shared__ double dyn_sh[];
-    __shared__ double red_sh[128];
-    __shared__ int flag_sh[2], any_sh;
-    Phaser<G, BLOCK> ph(D, dyn_sh, red_sh, flag_sh, &any_sh);
+    extern __shared__ __align__(128) unsigned char dyn_sh[];
+    __shared__ PhaseShared<BLOCK> psh;
+    Phaser<G, BLOCK, F> ph(D, dyn_sh, psh);
     if (blockIdx.x == 0 && threadIdx.x == 0)
         for (int s = 0; s < D.n_scenes; ++s) {
             SceneCtl c = ctl_load(D.ctl + s);
@@ -2985,12 +2844,13 @@ __global__ void __launch_bounds__(BLOCK, persist_min_blocks<BLOCK>()) k_force_pe
     if (!ph.barrier(-1)) return;
     ph.refresh();
     if (!ph.any(K_V_SETUP)) return;
-    if (FORCE == FORCE_ST && !ph.template run<M>(K_ST_DIV)) return;
-    if (!ph.template run<M>(K_V_SETUP)) return;
+    if constexpr (FORCE == FORCE_ST)
+        if (!ph.template run<K_ST_DIV, FORCE>()) return;
+    if (!ph.template run<K_V_SETUP, FORCE>()) return;
     while (ph.any(K_V_A)) {
-        if (!ph.template run<M>(K_V_A)) return;
+        if (!ph.template run<K_V_A, FORCE>()) return;
         if (!ph.any(K_V_B)) break;
-        if (!ph.template run<M>(K_V_B)) return;
+        if (!ph.template run<K_V_B, FORCE>()) return;
     }
     for (int t = blockIdx.x; t < D.n_tiles; t += gridDim.x) {
         const TileCtx T = tile_ctx<G>(D, t);
@@ -3007,12 +2867,11 @@ __global__ void __launch_bounds__(BLOCK, persist_min_blocks<BLOCK>()) k_force_pe
 }
 
 // The whole IP.solve of every scene in one persistent cooperative launch.
-template <int G, int BLOCK>
+template <int G, int BLOCK, int F>
 __global__ void __launch_bounds__(BLOCK, persist_min_blocks<BLOCK>()) k_ip_persistent(const Dev D) {
-    extern __shared__ double dyn_sh[];
-    __shared__ double red_sh[128];
-    __shared__ int flag_sh[2], any_sh;
-    Phaser<G, BLOCK> ph(D, dyn_sh, red_sh, flag_sh, &any_sh);
+    extern __shared__ __align__(128) unsigned char dyn_sh[];
+    __shared__ PhaseShared<BLOCK> psh;
+    Phaser<G, BLOCK, F> ph(D, dyn_sh, psh);
     // CTA 0 starts every scene's control block (reset_stats); the first
     // barrier publishes it
     if (blockIdx.x == 0 && threadIdx.x == 0)
@@ -3030,13 +2889,13 @@ __global__ void __launch_bounds__(BLOCK, persist_min_blocks<BLOCK>()) k_ip_persi
     if (!ph.barrier(-1)) return;
     ph.refresh();
     while (ph.any(K_PACK)) {
-        if (!ph.template run<MODE_IP>(K_PACK)) return;
+        if (!ph.template run<K_PACK>()) return;
         if (!ph.any(K_RHS)) break;
-        if (!ph.template run<MODE_IP>(K_RHS)) return;
+        if (!ph.template run<K_RHS>()) return;
         while (ph.any(K_CG_A)) {
-            if (!ph.template run<MODE_IP>(K_CG_A)) return;
+            if (!ph.template run<K_CG_A>()) return;
             if (!ph.any(K_CG_B)) break;
-            if (!ph.template run<MODE_IP>(K_CG_B)) return;
+            if (!ph.template run<K_CG_B>()) return;
         }
     }
     // epilogue (ip.py:394-404): v = d/dt for scenes that did not raise,
@@ -3054,12 +2913,12 @@ __global__ void __launch_bounds__(BLOCK, persist_min_blocks<BLOCK>()) k_ip_persi
             D.v[3 * p + 1] = s * d.y;
             D.v[3 * p + 2] = s * d.z;
         }
-        if (D.div_out) div_tile<G>(D, P, T, C.outer_it);
+        if (D.div_out) div_tile<G>(ph.rows, D, P, T, C);
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         for (int s = 0; s < D.n_scenes; ++s) {
             if (D.scenes[s].solver != SOLVER_IP) continue;
-            SceneCtl c = ctl_load(D.ctl + s);
+            SceneCtl c = ph.sc_sh[s];
             solve_account(c);
             D.ctl[s] = c;
         }
@@ -3068,12 +2927,11 @@ __global__ void __launch_bounds__(BLOCK, persist_min_blocks<BLOCK>()) k_ip_persi
 
 // The whole PRJ.solve of every PRJ scene in one persistent cooperative
 // launch: passes of head (no reduction) and tail (error, decision).
-template <int G, int BLOCK>
+template <int G, int BLOCK, int F>
 __global__ void __launch_bounds__(BLOCK, persist_min_blocks<BLOCK>()) k_prj_persistent(const Dev D) {
-    extern __shared__ double dyn_sh[];
-    __shared__ double red_sh[128];
-    __shared__ int flag_sh[2], any_sh;
-    Phaser<G, BLOCK> ph(D, dyn_sh, red_sh, flag_sh, &any_sh);
+    extern __shared__ __align__(128) unsigned char dyn_sh[];
+    __shared__ PhaseShared<BLOCK> psh;
+    Phaser<G, BLOCK, F> ph(D, dyn_sh, psh);
     if (blockIdx.x == 0 && threadIdx.x == 0)
         for (int s = 0; s < D.n_scenes; ++s)
             if (D.scenes[s].solver == SOLVER_PRJ) ctl_begin(D.scenes[s], D.ctl[s], SOLVER_PRJ);
@@ -3085,8 +2943,8 @@ __global__ void __launch_bounds__(BLOCK, persist_min_blocks<BLOCK>()) k_prj_pers
     if (!ph.barrier(-1)) return;
     ph.refresh();
     while (ph.any(K_PJ_HEAD)) {
-        if (!ph.template run<MODE_PRJ>(K_PJ_HEAD)) return;
-        if (!ph.template run<MODE_PRJ>(K_PJ_TAIL)) return;
+        if (!ph.template run<K_PJ_HEAD>()) return;
+        if (!ph.template run<K_PJ_TAIL>()) return;
     }
     for (int t = blockIdx.x; t < D.n_tiles; t += gridDim.x) {
         const TileCtx T = tile_ctx<G>(D, t);
@@ -3094,12 +2952,12 @@ __global__ void __launch_bounds__(BLOCK, persist_min_blocks<BLOCK>()) k_prj_pers
         if (P.solver != SOLVER_PRJ) continue;
         const SceneCtl& C = ph.sc_sh[T.sc];
         if (C.status == IVP_OK_ && T.lane == 0 && T.valid) pj_end_slot(D, P, T.i);
-        if (D.div_out) div_tile<G>(D, P, T, 0);
+        if (D.div_out) div_tile<G>(ph.rows, D, P, T, C);
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         for (int s = 0; s < D.n_scenes; ++s) {
             if (D.scenes[s].solver != SOLVER_PRJ) continue;
-            SceneCtl c = ctl_load(D.ctl + s);
+            SceneCtl c = ph.sc_sh[s];
             solve_account(c);
             D.ctl[s] = c;
         }

@@ -1,0 +1,229 @@
+// ivp_window.cuh -- the neighbour search of a few consecutive slots by one
+// warp: hit lists and the SPH sums over them, shared by the engine's neighbour
+// build and the allocation-free density.
+#pragma once
+#include <cmath>
+
+#include "ivp_device.cuh"
+
+namespace ivp {
+
+constexpr int kHits = 64;         // >= every cache_size the rows can hold
+constexpr int kMaxChunks = 16;    // window candidates / 32 of the filter pass
+constexpr int kOrdShift = 9;      // hit code: (range ordinal << 9) | window position (< 512)
+static_assert(kMaxChunks * 32 <= (1 << kOrdShift) && 18 << kOrdShift <= 65536, "hit codes are 16 bits");
+
+template <int SUB>
+struct BuildShared {
+    static constexpr int VMAX = SUB < 16 ? SUB : 16;   // runs with a kept window
+    static constexpr int kRunFill = 3;                 // a run takes in up to two more cells while it holds no more particles
+    float4 pos[SUB];
+    unsigned mask[kMaxChunks][SUB];
+    int delta[VMAX][18];                               // slot = delta[run][ordinal] + window position
+    int found[SUB];                                    // hits of each particle (not capped); -1: scan it alone
+    unsigned short code[kMaxChunks * 32];
+    unsigned short hit[kHits][SUB];
+};
+
+// Largest float r2 with sqrtf(r2) < h: `r2 <= r2_max` is the strict `|r| < h` test
+// (IEEE sqrt is monotone and correctly rounded on host and device alike).
+inline float strict_r2_max(float h) {
+    float t = h * h;
+    while (std::sqrt(t) >= h) t = std::nextafter(t, 0.0f);
+    while (std::sqrt(std::nextafter(t, INFINITY)) < h) t = std::nextafter(t, INFINITY);
+    return t;
+}
+
+// What the scan of a cell's window needs (one scene of an engine, or the grid
+// of ivp_density_aii_noalloc).
+struct WindowGrid {
+    const int* cell_start;  // of the scene's keys: dynamic cells, then static cells
+    const float4* xm;
+    int ncell, dims[3];
+    float r2_max;
+};
+
+// Lane q < 18: the q-th slot range of the window of cells (cx .. cx1, cy, cz).
+__device__ __forceinline__ void window_range(const WindowGrid& W, int cx, int cx1, int cy, int cz, int q, int& b,
+                                             int& len) {
+    b = len = 0;
+    const int rr = q >> 1;
+    const int z = cz + rr / 3 - 1, y = cy + rr % 3 - 1;
+    if (q < 18 && z >= 0 && z < W.dims[2] && y >= 0 && y < W.dims[1]) {
+        const int x0 = cx > 0 ? cx - 1 : 0, x1 = cx1 < W.dims[0] - 1 ? cx1 + 1 : W.dims[0] - 1;
+        const int* cs = W.cell_start + ((q & 1) ? W.ncell : 0) + (z * W.dims[1] + y) * W.dims[0];
+        b = __ldg(cs + x0);
+        len = __ldg(cs + x1 + 1) - b;
+    }
+}
+
+// Filter pass of one warp over slots i0 .. i0 + n - 1 (n <= SUB).  Lane l < n
+// passes its particle's position and cell; it returns the lane's run, and leaves
+// every particle's hit count and list in S.
+template <int SUB>
+__device__ __forceinline__ int filter_hits(const WindowGrid& W, BuildShared<SUB>& S, int i0, int n, float4 xi,
+                                             int3 cell, int cap) {
+    const int lane = threadIdx.x & 31;
+    const unsigned le = 0xffffffffu >> (31 - lane);
+    if (lane < n) {
+        S.pos[lane] = xi;
+        S.found[lane] = 0;
+    }
+    const int row = lane < n ? cell.z * W.dims[1] + cell.y : -1;
+    int mine = 0;
+    __syncwarp();
+    for (int first = 0, run = 0; first < n; ++run) {
+        const int cx = __shfl_sync(0xffffffffu, cell.x, first);
+        const int cy = __shfl_sync(0xffffffffu, cell.y, first);
+        const int cz = __shfl_sync(0xffffffffu, cell.z, first);
+        const bool after = lane >= first && row == cz * W.dims[1] + cy;
+        int ext = 0;
+        int np = __popc(__ballot_sync(0xffffffffu, after && cell.x == cx));
+        for (int e = 1; e <= 2 && np < BuildShared<SUB>::kRunFill; ++e) {
+            const int more = __popc(__ballot_sync(0xffffffffu, after && cell.x <= cx + e));
+            if (more > BuildShared<SUB>::kRunFill) break;
+            np = more;
+            ext = e;
+        }
+        int b, len;
+        window_range(W, cx, cx + ext, cy, cz, lane, b, len);
+        int incl = len;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += t;
+        }
+        const int L = __shfl_sync(0xffffffffu, incl, 31);
+        if (L > kMaxChunks * 32 || run >= BuildShared<SUB>::VMAX) {
+            // a crowded window, or particles scattered over many cells: each
+            // is scanned on its own by the whole warp
+            if (lane < np) S.found[first + lane] = -1;
+            first += np;
+            continue;
+        }
+        const int off = incl - len;
+        const unsigned some = __ballot_sync(0xffffffffu, len > 0);
+        if (len > 0) S.delta[run][__popc(some & le) - 1] = b - off;
+        const int self = __shfl_sync(0xffffffffu, b - off, 8);  // range 8: the run's own cell row
+        __syncwarp();
+        int ord = -1;  // last range begun before the chunk
+        auto chunk = [&](int c) {
+            const unsigned rel = (unsigned)(off - 32 * c);
+            const unsigned starts = __reduce_or_sync(0xffffffffu, (len > 0 && rel < 32u) ? 1u << rel : 0u);
+            const int o = ord + __popc(starts & le);
+            ord += __popc(starts);
+            const int v = 32 * c + lane;
+            float4 x = make_float4(__int_as_float(0x7fc00000), 0.f, 0.f, 0.f);  // past the end: never within h
+            if (v < L) {
+                S.code[v] = (unsigned short)((o << kOrdShift) | v);
+                x = __ldg(W.xm + (S.delta[run][o] + v));
+            }
+            return x;
+        };
+        const int nch = (L + 31) >> 5;
+        float4 xn = chunk(0);
+        for (int c = 0; c < nch; ++c) {
+            const float4 xj = xn;
+            if (c + 1 < nch) xn = chunk(c + 1);
+#pragma unroll 4
+            for (int p = 0; p < np; ++p) {
+                const float4 xp = S.pos[first + p];
+                const float3 r = make_float3(xp.x - xj.x, xp.y - xj.y, xp.z - xj.z);
+                const unsigned ball = __ballot_sync(0xffffffffu, norm2_rn(r) <= W.r2_max);
+                if (lane == 0) S.mask[c][first + p] = ball;
+            }
+        }
+        __syncwarp();
+        if (lane >= first && lane < first + np) mine = run;
+        {
+            // expand: lane (c0, p) takes chunks c0, c0 + nc, ... of particle p
+            const int sh = np <= 8 ? 3 : np <= 16 ? 4 : 5;
+            const int p = lane & ((1 << sh) - 1), c0 = lane >> sh, nc = 32 >> sh;
+            const int vself = i0 + first + p - self;  // the particle's own window position
+            int count = 0;
+            for (int cb = 0; cb < nch; cb += nc) {
+                const int c = cb + c0;
+                unsigned m = (p < np && c < nch) ? S.mask[c][first + p] : 0u;
+                if (c == (vself >> 5)) m &= ~(1u << (vself & 31));
+                int sum = __popc(m);
+                const int own = sum;
+#pragma unroll
+                for (int o = 8; o < 32; o <<= 1) {
+                    const int t = __shfl_up_sync(0xffffffffu, sum, o);
+                    if (o >= (1 << sh) && lane >= o) sum += t;
+                }
+                int at = count + sum - own;
+                count += __shfl_sync(0xffffffffu, sum, p | (32 - (1 << sh)));
+                while (m) {
+                    const int bit = __ffs(m) - 1;
+                    m &= m - 1u;
+                    if (at < cap) S.hit[at][first + p] = S.code[32 * c + bit];
+                    ++at;
+                }
+            }
+            if (c0 == 0 && p < np) S.found[first + p] = count;
+            __syncwarp();
+        }
+        first += np;
+    }
+    return mine;
+}
+
+// Sums of one particle over its hits.  One reciprocal mass is kept: the
+// dynamic neighbours of a particle nearly always have the same mass.
+struct HitSums {
+    float rho = 0.0f, aii = 0.0f, m_of = 0.0f, inv_m = 0.0f;
+    float3 jii = make_float3(0.0f, 0.0f, 0.0f);
+};
+
+// The pair terms of hit j at squared distance r2 (sph_kernel.py:8-61) onto the
+// sums; returns J_ij and its weight.
+__device__ __forceinline__ float3 hit_terms(float3 r, float r2, float mj, bool dynamic, float h, float inv_h,
+                                            float spk, float ck, HitSums& s, float* weight) {
+    // spiky gradient (sph_kernel.py:52-61): -k (h - |r|)^2 r / |r|
+    const float rn = sqrtf(r2);
+    const float rc = rn < 1e-6f ? 1e-6f : rn;
+    const float t = h - rc;
+    const float sg = -spk * (t * t);
+    const float ir = __frcp_rn(rc);
+    const float w = mj * (sg * ir);
+    const float3 J = make_float3(__fmul_rn(w, r.x), __fmul_rn(w, r.y), __fmul_rn(w, r.z));
+    s.rho += mj * cubic_Wq(rn * inv_h, ck);
+    if (dynamic) {
+        if (mj != s.m_of) {
+            s.m_of = mj;
+            s.inv_m = __frcp_rn(mj);
+        }
+        s.aii += dot3(J, J) * s.inv_m;
+    }
+    s.jii = sub3(s.jii, J);
+    *weight = w;
+    return J;
+}
+
+template <int LANES>
+__device__ __forceinline__ void sum_lanes(HitSums& s) {
+#pragma unroll
+    for (int o = LANES / 2; o > 0; o >>= 1) {
+        s.rho += __shfl_xor_sync(0xffffffffu, s.rho, o);
+        s.aii += __shfl_xor_sync(0xffffffffu, s.aii, o);
+        s.jii.x += __shfl_xor_sync(0xffffffffu, s.jii.x, o);
+        s.jii.y += __shfl_xor_sync(0xffffffffu, s.jii.y, o);
+        s.jii.z += __shfl_xor_sync(0xffffffffu, s.jii.z, o);
+    }
+}
+
+// The sums of particles p0 .. p0 + 3, in the eight lanes of each, to the lanes
+// p0 .. p0 + 3.
+__device__ __forceinline__ void own_sums(const HitSums& a, int p0, HitSums& s) {
+    const int lane = threadIdx.x & 31, from = ((lane - p0) * 8) & 31;
+    HitSums g;
+    g.rho = __shfl_sync(0xffffffffu, a.rho, from);
+    g.aii = __shfl_sync(0xffffffffu, a.aii, from);
+    g.jii.x = __shfl_sync(0xffffffffu, a.jii.x, from);
+    g.jii.y = __shfl_sync(0xffffffffu, a.jii.y, from);
+    g.jii.z = __shfl_sync(0xffffffffu, a.jii.z, from);
+    if (lane >= p0 && lane < p0 + 4) s = g;
+}
+
+}  // namespace ivp

@@ -35,6 +35,7 @@
 #include "../../include/ivp.h"
 #include "ivp_device.cuh"
 #include "ivp_scan.cuh"
+#include "ivp_window.cuh"
 
 namespace ivp {
 // the engine's thread-local error text (ivp_last_error), set in ivp_engine.cu
@@ -44,12 +45,7 @@ void set_last_error(const std::string& msg);
 namespace {
 
 using ivp::cell_coord;
-using ivp::cubic_W;
 using ivp::dot3;
-using ivp::f3;
-using ivp::scale3;
-using ivp::spiky_w;
-using ivp::sub3;
 
 constexpr int kMaxParticles = IVP_NOALLOC_MAX_PARTICLES;
 constexpr int kMaxKeys = 2 * IVP_NOALLOC_MAX_CELLS;
@@ -75,7 +71,7 @@ Scratch* g_scratch_addr[kMaxDevices] = {};
 struct Grid {
     int dims[3];
     int ncell;
-    float cell_inv, h, cubic_k, spiky_k, W0;
+    float cell_inv, h, inv_h, cubic_k, spiky_k, W0, r2_max;
     int cap;
 };
 
@@ -114,60 +110,99 @@ __global__ void na_order(const float* __restrict__ x, const float* __restrict__ 
 // dynamic particle over its first `cap` neighbours |x_i - x_j| < h, j != i
 // (neighbour_search.py:10-51), in the same candidate order as the engine's
 // neighbour build, but without storing the lists.  Static particles get k = 0.
-__global__ void na_density_aii(int n, Grid g, Scratch* S, float* __restrict__ density, float* __restrict__ kdiag) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+//
+// One warp per eight slots, as in the engine's build for small scenes: a thread
+// per particle walked 270 candidates one after another, on 176 CTAs of 256
+// threads for 40,000 particles (99 us), and left most of the chip waiting.
+constexpr int kSub = 8, kWarps = 2;
+
+__global__ void __launch_bounds__(32 * kWarps) na_density_aii(int n, Grid g, Scratch* S, float* __restrict__ density,
+                                                              float* __restrict__ kdiag) {
+    __shared__ ivp::BuildShared<kSub> sh[kWarps];
+    const int lane = threadIdx.x & 31;
+    ivp::BuildShared<kSub>& B = sh[threadIdx.x >> 5];
+    const int i0 = (blockIdx.x * kWarps + (threadIdx.x >> 5)) * kSub;
+    if (i0 >= n) return;  // warp-uniform; the kernel has no CTA barrier
     const int n_dyn = S->cell_start[g.ncell];
-    const int p = S->pid[i];
-    if (i >= n_dyn) {
-        kdiag[p] = 0.0f;
-        return;
+    if (lane < kSub && i0 + lane < n && i0 + lane >= n_dyn) kdiag[S->pid[i0 + lane]] = 0.0f;
+    const int m = min(kSub, n_dyn - i0);
+    if (m <= 0) return;
+    ivp::WindowGrid W;
+    W.cell_start = S->cell_start;
+    W.xm = S->xm;
+    W.ncell = g.ncell;
+    for (int a = 0; a < 3; ++a) W.dims[a] = g.dims[a];
+    W.r2_max = g.r2_max;
+    float4 xl = make_float4(0.f, 0.f, 0.f, 0.f);
+    int3 cell = make_int3(0, 0, 0);
+    int pid = 0;
+    if (lane < m) {
+        xl = W.xm[i0 + lane];
+        pid = S->pid[i0 + lane];
+        cell = make_int3(cell_coord(xl.x, g.cell_inv, g.dims[0]), cell_coord(xl.y, g.cell_inv, g.dims[1]),
+                         cell_coord(xl.z, g.cell_inv, g.dims[2]));
     }
-    const float4 xi4 = S->xm[i];
-    const float3 xi = f3(xi4);
-    const float mi = xi4.w;
-    const float h = g.h;
-    const int cx = cell_coord(xi.x, g.cell_inv, g.dims[0]);
-    const int cy = cell_coord(xi.y, g.cell_inv, g.dims[1]);
-    const int cz = cell_coord(xi.z, g.cell_inv, g.dims[2]);
-    float rho = 0.0f;
-    rho = rho + mi * g.W0;
-    float aii = 0.0f;
-    float3 jii = make_float3(0.0f, 0.0f, 0.0f);
-    int cnt = 0;
-    const int x0 = cx > 0 ? cx - 1 : 0;
-    const int x1 = cx < g.dims[0] - 1 ? cx + 1 : g.dims[0] - 1;
-    for (int dz = -1; dz <= 1; ++dz) {
-        const int z = cz + dz;
-        if (z < 0 || z >= g.dims[2]) continue;
-        for (int dy = -1; dy <= 1; ++dy) {
-            const int yy = cy + dy;
-            if (yy < 0 || yy >= g.dims[1]) continue;
-            const int cb = (z * g.dims[1] + yy) * g.dims[0];
-            for (int pass = 0; pass < 2; ++pass) {
-                const int kb = (pass ? g.ncell : 0) + cb;
-                const int jb = S->cell_start[kb + x0], je = S->cell_start[kb + x1 + 1];
-                for (int j = jb; j < je; ++j) {
-                    if (j == i) continue;
-                    const float4 xj4 = S->xm[j];
-                    const float3 r = sub3(xi, f3(xj4));
-                    const float rn = sqrtf(dot3(r, r));
-                    if (rn < h && cnt < g.cap) {
-                        const float w = spiky_w(rn, h, g.spiky_k);
-                        const float mj = xj4.w;
-                        rho += mj * cubic_W(rn, h, g.cubic_k);
-                        const float3 J = scale3(mj, scale3(w, r));
-                        if (j < n_dyn) aii += dot3(J, J) * (1.0f / mj);
-                        jii = sub3(jii, J);
-                        ++cnt;
-                    }
-                }
+    const int run = ivp::filter_hits<kSub>(W, B, i0, m, xl, cell, ivp::kHits);
+    __syncwarp();
+    ivp::HitSums s;  // lane p's own particle
+    const int found = lane < m ? B.found[lane] : 0;
+    // more hits than a list holds (a cache_size above it only), or a window
+    // that does not fit the filter: the whole warp on one particle
+    const unsigned alone = __ballot_sync(0xffffffffu, found < 0 || (found > ivp::kHits && g.cap > ivp::kHits));
+    for (int p0 = 0; p0 < m; p0 += 4) {
+        // eight lanes per particle
+        const int p = p0 + (lane >> 3), q = min(p, m - 1);
+        const int n_hit = p < m ? min(min(B.found[p], ivp::kHits), g.cap) : 0;
+        const int* delta = B.delta[__shfl_sync(0xffffffffu, run, q)];
+        const float4 xi = B.pos[q];
+        ivp::HitSums a;
+        for (int k = lane & 7; k < n_hit; k += 8) {
+            const int code = B.hit[k][p];
+            const int j = delta[code >> ivp::kOrdShift] + (code & ((1 << ivp::kOrdShift) - 1));
+            const float4 xj = __ldg(W.xm + j);
+            const float3 r = make_float3(xi.x - xj.x, xi.y - xj.y, xi.z - xj.z);
+            float w;
+            ivp::hit_terms(r, ivp::norm2_rn(r), xj.w, j < n_dyn, g.h, g.inv_h, g.spiky_k, g.cubic_k, a, &w);
+        }
+        __syncwarp();
+        ivp::sum_lanes<8>(a);
+        ivp::own_sums(a, p0, s);
+    }
+    for (unsigned left = alone; left; left &= left - 1u) {
+        const int p = __ffs(left) - 1, i = i0 + p;
+        const float4 xi = B.pos[p];
+        int b, len, at = 0;
+        ivp::window_range(W, cell_coord(xi.x, g.cell_inv, g.dims[0]), cell_coord(xi.x, g.cell_inv, g.dims[0]),
+                          cell_coord(xi.y, g.cell_inv, g.dims[1]), cell_coord(xi.z, g.cell_inv, g.dims[2]), lane, b, len);
+        ivp::HitSums a;
+        for (int q = 0; q < 18; ++q) {
+            const int jb = __shfl_sync(0xffffffffu, b, q), c = __shfl_sync(0xffffffffu, len, q);
+            for (int base = 0; base < c; base += 32) {
+                const int j = jb + base + lane;
+                float4 xj = xi;
+                if (base + lane < c) xj = __ldg(W.xm + j);
+                const float3 r = make_float3(xi.x - xj.x, xi.y - xj.y, xi.z - xj.z);
+                const float r2 = ivp::norm2_rn(r);
+                const bool in = base + lane < c && j != i && r2 <= W.r2_max;
+                const unsigned ball = __ballot_sync(0xffffffffu, in);
+                float w;
+                if (in && at + __popc(ball & ((1u << lane) - 1u)) < g.cap)
+                    ivp::hit_terms(r, r2, xj.w, j < n_dyn, g.h, g.inv_h, g.spiky_k, g.cubic_k, a, &w);
+                at += __popc(ball);
             }
         }
+        ivp::sum_lanes<32>(a);
+        if (lane == p) s = a;
     }
-    aii += dot3(jii, jii) * (1.0f / mi);
-    density[p] = rho;
-    kdiag[p] = 1.0f / (aii + 1e-3f);
+    if (lane < m) {
+        const float mi = xl.w;
+        float rho = 0.0f;
+        rho = rho + mi * g.W0;
+        rho += s.rho;
+        const float aii = s.aii + dot3(s.jii, s.jii) * __frcp_rn(mi);
+        density[pid] = rho;
+        kdiag[pid] = __frcp_rn(aii + 1e-3f);
+    }
 }
 
 // Every failure leaves its reason where ivp_last_error() reads it.
@@ -214,6 +249,8 @@ extern "C" int ivp_density_aii_noalloc(const float* x, const float* m, const int
     g.ncell = (int)ncell;
     g.h = h;
     g.cell_inv = 1.0f / h;
+    g.inv_h = 1.0f / h;
+    g.r2_max = ivp::strict_r2_max(h);
     float k = 8.0f / 3.14159265359f;
     k = k / (h * h * h);
     g.cubic_k = k;
@@ -267,7 +304,8 @@ extern "C" int ivp_density_aii_noalloc(const float* x, const float* m, const int
     if (st == IVP_OK) st = launch((const void*)ivp::k_scan_add, nsb, ivp::SCAN_BLOCK, a_scan2, s, "scan_add");
     if (st == IVP_OK) st = launch((const void*)na_place, nb, B, a_place, s, "na_place");
     if (st == IVP_OK) st = launch((const void*)na_order, nb, B, a_order, s, "na_order");
-    if (st == IVP_OK) st = launch((const void*)na_density_aii, nb, B, a_dens, s, "na_density_aii");
+    if (st == IVP_OK) st = launch((const void*)na_density_aii, (n + kSub * kWarps - 1) / (kSub * kWarps), 32 * kWarps, a_dens, s,
+                                   "na_density_aii");
     if (st != IVP_OK) return st;
     return IVP_OK;
 }

@@ -370,24 +370,22 @@ int emit_build_impl(ivp_engine* e, Launcher& L, bool with_advect) {
             CK(cudaGraphConditionalHandleCreate(&h_fix, L.graph, 0, cudaGraphCondAssignDefault));
             copy.h_fix = (unsigned long long)h_fix;
         }
-        if (e->opt.build_kernel == 2) {
-            // warps of eight slots, or of a slice of rows where that is more
-            const int sub = std::max(8, 32 / e->G);
-            const int warps = e->n_tiles * blocks_for(e->T, sub);
-            int T = e->T;
-            void* args[] = {&copy, &T};
-            CKS(L.kernel(IVP_K_NBR_BUILD,
-                         sub == 8    ? (const void*)k_nbr_build<8>
-                         : sub == 16 ? (const void*)k_nbr_build<16>
-                                     : (const void*)k_nbr_build<32>,
-                         dim3(blocks_for(warps, kBuildWarps)), dim3(32 * kBuildWarps), args));
-        } else {
-            // one thread per dynamic particle, one CTA per tile
-            const int nt = std::max(e->T, 32);
-            void* args[] = {&copy};
-            CKS(L.kernel(IVP_K_NBR_BUILD, (const void*)k_nbr_build_tpp, dim3(e->n_tiles), dim3(nt), args,
-                         sizeof(unsigned short) * kTppHits * nt));
-        }
+        // Build kernel 1 sums the density in list order: eight slots a warp at
+        // 4 and 8 lanes per particle, 32 at 1 and 2 (many particles: fewer
+        // windows walked).  Build kernel 2 does not; its warps take eight slots
+        // or a slice of rows.  A warp never takes less than a slice, whose rows
+        // it fills up together.
+        const bool ordered = e->opt.build_kernel != 2;
+        const int sub = e->G >= 4 ? 8 : ordered || e->G == 1 ? 32 : 16;
+        const void* fn = sub == 32   ? (const void*)k_nbr_build<32, true>
+                         : sub == 16 ? (const void*)k_nbr_build<16, false>
+                         : ordered   ? (const void*)k_nbr_build<8, true>
+                                     : (const void*)k_nbr_build<8, false>;
+        const int warps = e->n_tiles * blocks_for(e->T, sub);
+        int T = e->T;
+        void* args[] = {&copy, &T};
+        CKS(L.kernel(IVP_K_NBR_BUILD, fn,
+                     dim3(blocks_for(warps, kBuildWarps)), dim3(32 * kBuildWarps), args));
         if (L.graph) {
             cudaGraph_t body;
             CKS(add_conditional(L.graph, L, h_fix, cudaGraphCondTypeIf, &body));

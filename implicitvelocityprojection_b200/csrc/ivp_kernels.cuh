@@ -448,8 +448,7 @@ __global__ void k_order(const Dev D) {
 // diagonal k = 1/(Aii + 1e-3) (pressure_base.py:49-87) and the constraint
 // c = rho - rho0 (pressure_base.py:169-184).
 //
-// One warp takes SUB consecutive dynamic slots (8, or a slice of rows where that
-// is more) and works in two passes.
+// One warp takes SUB consecutive dynamic slots and works in two passes.
 //
 // Filter: the slots are sorted by cell, so the warp's particles are a few runs
 // of one cell each (or of a few thinly filled x-adjacent cells), and the
@@ -457,19 +456,19 @@ __global__ void k_order(const Dev D) {
 // ranges (rows dz outer, dy inner; dynamic then static slots of the x-adjacent
 // cells), walked end to end in chunks of 32: a lane holds one candidate of the
 // chunk, all lanes test it against one particle of the run after another, and
-// one ballot per particle and chunk is the whole result.  The ballots are then
-// expanded into each particle's hit list (16 bits a hit: the range's ordinal and
-// the window position), in the sequential candidate order, so the first
-// cache_size kept are those of the sequential scan.
+// one ballot per particle and chunk is the whole result.
 //
-// Dense pass: eight lanes per particle walk its list and form the row entry,
-// density and Aii terms of every hit.
-//
-// For scenes of few particles per SM, which wait for one warp's chain of loads:
-// no staging and no CTA barrier before the first test.  Against one CTA per run
-// of eight cells with its candidates staged in shared memory: 8,192 particles
-// 33 us instead of 35, 31,007 particles 47 us instead of 52 (768: 27 and 25).
-constexpr int kBuildWarps = 2;  // warps per CTA
+// Dense pass: the ballots' bits, in window order, are a particle's hits in the
+// sequential candidate order, so the first cache_size kept are those of the
+// sequential scan.
+//   SUB = 32: each lane walks the bits of its own particle.
+//   SUB = 8, or a slice of rows where that is more: the bits are expanded into
+//   hit lists and eight lanes share a particle; more warps with shorter chains
+//   of loads.
+// ORDERED adds the density in list order, as the reference does (SUB = 32 does by
+// its nature): rho - rho0 cancels all but the last digits of the sum, and a
+// constraint near zero falls on one side of the operator's switch or the other.
+constexpr int kBuildWarps = 1;  // warps per CTA: they share nothing, and a CTA's slot is free as soon as its warp is done
 
 // All hits of one particle by the whole warp, straight from its window: for
 // windows that do not fit the filter pass.  Every lane returns the sums;
@@ -513,7 +512,7 @@ __device__ __forceinline__ int scan_alone(const WindowGrid& W, int* list, int i,
     return found;
 }
 
-template <int SUB>
+template <int SUB, bool ORDERED>
 __global__ void __launch_bounds__(32 * kBuildWarps) k_nbr_build(const Dev D, int tile_size) {
     __shared__ BuildShared<SUB> sh[kBuildWarps];
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -555,35 +554,85 @@ __global__ void __launch_bounds__(32 * kBuildWarps) k_nbr_build(const Dev D, int
         cell = cell_of(xl);
         material = D.material[pid];
     }
-    const int mine = filter_hits<SUB>(W, S, i0, n, xl, cell, cap);
+    const RunOf mine = filter_hits<SUB>(W, S, i0, n, xl, cell, cap);
     __syncwarp();
     // the row entry, density and Aii terms of hit k of slot i
     auto take = [&](int i, int k, int j, float4 xi, float4 xj, float3 r, float r2, HitSums& s) {
-        float w;
-        const float3 J = hit_terms(r, r2, xj.w, j < dyn_end, h, inv_h, spk, ck, s, &w);
+        float w, Wj;
+        const float3 J = hit_terms(r, r2, xj.w, j < dyn_end, h, inv_h, spk, ck, s, &w, &Wj);
         put_entry(D, P.row_base + (i - P.s_begin), k, j, J, w);
+        return Wj;
     };
     HitSums s;      // lane p's own particle
     int found = lane < n ? S.found[lane] : 0;
     const unsigned alone = __ballot_sync(0xffffffffu, found < 0);
-    {
+    if constexpr (!BuildShared<SUB>::kLists) {
+        // each lane walks the bits of its own particle and sums in list order
+        const int i = i0 + lane;
+        const int* delta = S.delta[mine.run];
+        const int2* starts = S.starts[mine.run];
+        const int chunks = lane < n && found == 0 ? mine.chunks : 0;
+        unsigned m = chunks > 0 ? S.mask[0][lane] : 0u;
+        int c = 0;
+        // slot of the next candidate the filter let through, -1 at the end
+        auto next = [&]() {
+            while (m == 0u && c + 1 < chunks) m = S.mask[++c][lane];
+            if (m == 0u) return -1;
+            const int bit = __ffs(m) - 1;
+            m &= m - 1u;
+            const int2 st = starts[c];
+            return delta[st.y + __popc((unsigned)st.x & (0xffffffffu >> (31 - bit)))] + 32 * c + bit;
+        };
+        // two at a time, so that their position loads overlap
+        for (;;) {
+            int j[2];
+            float4 xj[2];
+            j[0] = next();
+            if (j[0] < 0) break;
+            j[1] = next();
+#pragma unroll
+            for (int u = 0; u < 2; ++u) xj[u] = __ldg(D.xm + (j[u] < 0 ? i : j[u]));
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const float3 r = make_float3(xl.x - xj[u].x, xl.y - xj[u].y, xl.z - xj[u].z);
+                const float r2 = norm2_rn(r);
+                if (j[u] >= 0 && j[u] != i && r2 <= W.r2_max) {
+                    if (found < cap) take(i, found, j[u], xl, xj[u], r, r2, s);
+                    ++found;
+                }
+            }
+        }
+    } else {
         // eight lanes per particle, four particles at a time
         const int sub = lane & 7;
         for (int p0 = 0; p0 < n; p0 += 4) {
             const int p = p0 + (lane >> 3);
             const int n_hit = p < n ? min(S.found[p], cap) : 0;
-            const int* delta = S.delta[__shfl_sync(0xffffffffu, mine, min(p, n - 1))];
+            const int* delta = S.delta[__shfl_sync(0xffffffffu, mine.run, min(p, n - 1))];
             const float4 xi = S.pos[min(p, n - 1)];
             HitSums a;
-            for (int k = sub; k < n_hit; k += 8) {
-                const int code = S.hit[k][p];
-                const int j = delta[code >> kOrdShift] + (code & ((1 << kOrdShift) - 1));
-                const float4 xj = __ldg(D.xm + j);
-                const float3 r = make_float3(xi.x - xj.x, xi.y - xj.y, xi.z - xj.z);
-                take(i0 + p, k, j, xi, xj, r, norm2_rn(r), a);
+            float rho = 0.0f;
+            for (int k0 = 0; k0 < n_hit; k0 += 8) {  // the same in a particle's lanes
+                const int k = k0 + sub;
+                float mj = 0.0f, Wj = 0.0f;
+                if (k < n_hit) {
+                    const int code = S.hit[k][p];
+                    const int j = delta[code >> kOrdShift] + (code & ((1 << kOrdShift) - 1));
+                    const float4 xj = __ldg(D.xm + j);
+                    const float3 r = make_float3(xi.x - xj.x, xi.y - xj.y, xi.z - xj.z);
+                    Wj = take(i0 + p, k, j, xi, xj, r, norm2_rn(r), a);
+                    mj = xj.w;
+                }
+                if constexpr (ORDERED) {
+                    const unsigned group = 0xffu << (lane & 24);
+#pragma unroll
+                    for (int q = 0; q < 8; ++q)
+                        rho = __fmaf_rn(__shfl_sync(group, mj, (lane & 24) + q), __shfl_sync(group, Wj, (lane & 24) + q), rho);
+                }
             }
             __syncwarp();
             sum_lanes<8>(a);
+            if constexpr (ORDERED) a.rho = rho;
             own_sums(a, p0, s);
         }
     }
@@ -631,168 +680,6 @@ __global__ void __launch_bounds__(32 * kBuildWarps) k_nbr_build(const Dev D, int
     }
     pairs = __reduce_add_sync(0xffffffffu, pairs);
     if (lane == 0 && pairs) atomicAdd(&D.pairs[sc], (unsigned long long)pairs);
-}
-
-// Neighbour lists, density, Aii, k, c and 1/rho of every dynamic particle,
-// one thread per particle (one CTA per tile of dynamic slots).  The thread
-// walks its 27-cell window in the same sequential candidate order as
-// k_nbr_build -- (y, z) rows with dz outer and dy inner, in each row the
-// dynamic then the static slots of the x-adjacent cells, slots ascending --
-// so it keeps the same first cache_size hits.  Two passes: the filter loop
-// only appends each kept hit to the thread's list in shared memory as 16 bits
-// (which of the 18 slot ranges, and the offset in it; hit k of thread t at
-// [k * blockDim + t], so two neighbouring threads share a 4-byte bank word:
-// at most 2-way conflicts), then a dense pass rebuilds each hit's
-// slot and computes its row entry, density and Aii terms.  The filter, which
-// runs for every candidate, stays short even though the lanes of a warp hit
-// on different iterations; the small list leaves most of L1 to the candidate
-// positions that neighbouring threads (neighbouring slots) share.  A range
-// offset that does not fit the 10 bits (more than 1,023 slots in three cells
-// of one row) sets the scene's fix-up failure flag, so its IP solve stops
-// with IVP_ERR_NBR_OVERFLOW instead of using a wrong list.
-constexpr int kTppMaxThreads = 128;
-constexpr int kTppHits = 64;  // >= every cache_size (the row stride caps it)
-constexpr int kTppOffBits = 10;
-
-__global__ void __launch_bounds__(kTppMaxThreads) k_nbr_build_tpp(const Dev D) {
-    extern __shared__ unsigned short hit_q[];
-    const int nt = blockDim.x;
-    const int4 tile = __ldg(D.tiles + blockIdx.x);
-    const int sc = tile.x;
-    const SceneParams& P = D.scenes[sc];
-    const int tid = threadIdx.x;
-    const int i = tile.y + tid;
-    const bool act = i < tile.z;
-    int n_hit = 0;
-    if (act) {
-        const float4 xi4 = D.xm[i];
-        const float3 xi = f3(xi4);
-        const int dimx = P.dims[0];
-        const int cx = cell_coord(xi.x, P.cell_inv, dimx);
-        const int cy = cell_coord(xi.y, P.cell_inv, P.dims[1]);
-        const int cz = cell_coord(xi.z, P.cell_inv, P.dims[2]);
-        const int x0 = cx > 0 ? cx - 1 : 0, x1 = cx < dimx - 1 ? cx + 1 : dimx - 1;
-        const float r2max = P.r2_max;
-        const int cap = min(min(P.cache, D.stride), kTppHits);
-        int found = 0;
-        bool too_wide = false;
-        // filter, one dz plane (six slot ranges) at a time: the twelve range
-        // bounds of a plane load together, so a thread waits on three rounds
-        // of cell-start loads instead of eighteen
-        for (int dz = 0; dz < 3; ++dz) {
-            const int z = cz + dz - 1;
-            int rb[6], re[6];
-#pragma unroll
-            for (int u = 0; u < 6; ++u) {
-                const int y = cy + (u >> 1) - 1, pass = u & 1;
-                rb[u] = re[u] = 0;
-                if (z >= 0 && z < P.dims[2] && y >= 0 && y < P.dims[1]) {
-                    const int kb = P.key_base + (pass ? P.ncell : 0) + (z * P.dims[1] + y) * dimx;
-                    rb[u] = __ldg(D.cell_start + kb + x0);
-                    re[u] = __ldg(D.cell_start + kb + x1 + 1);
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < 6; ++u) {
-                const int q = dz * 6 + u, jb = rb[u], je = re[u];
-#pragma unroll 4
-                for (int j = jb; j < je; ++j) {
-                    const float3 r = sub3(xi, f3(__ldg(D.xm + j)));
-                    if (j != i && norm2_rn(r) <= r2max) {
-                        const int off = j - jb;
-                        too_wide |= off >= (1 << kTppOffBits);
-                        if (found < cap) hit_q[found * nt + tid] = (unsigned short)((q << kTppOffBits) | (off & 1023));
-                        ++found;
-                    }
-                }
-            }
-        }
-        n_hit = min(found, cap);
-        if (too_wide) D.fix_fail[sc] = 1;
-        // dense pass: the build's arithmetic for every kept hit, in order;
-        // two hits at a time, so their position loads are in flight together
-        // (four: 80 registers, slower on the larger scenes)
-        const float h = P.h, inv_h = P.inv_h, spk = P.spiky_k, ck = P.cubic_k;
-        const int dyn_end = P.s_dyn_end;
-        const int row = P.row_base + (i - P.s_begin);
-        float rho = 0.0f, aii = 0.0f;
-        float3 jii = make_float3(0.0f, 0.0f, 0.0f);
-        int q_cur = -1, jb_cur = 0;
-        for (int k0 = 0; k0 < n_hit; k0 += 2) {
-            int jj[2];
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                jj[u] = i;
-                if (k0 + u < n_hit) {
-                    const unsigned hq = hit_q[(k0 + u) * nt + tid];
-                    const int q = (int)(hq >> kTppOffBits);
-                    if (q != q_cur) {  // hits come in range order: one cell-start load per range
-                        q_cur = q;
-                        const int rr = q >> 1, pass = q & 1;
-                        const int z = cz + rr / 3 - 1, y = cy + rr % 3 - 1;
-                        jb_cur = __ldg(D.cell_start + P.key_base + (pass ? P.ncell : 0) + (z * P.dims[1] + y) * dimx + x0);
-                    }
-                    jj[u] = jb_cur + (int)(hq & 1023u);
-                }
-            }
-            float4 xq[2];
-#pragma unroll
-            for (int u = 0; u < 2; ++u) xq[u] = __ldg(D.xm + jj[u]);
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                const int k = k0 + u;
-                if (k >= n_hit) break;
-                const int j = jj[u];
-                const float4 xj4 = xq[u];
-                const float3 r = sub3(xi, f3(xj4));
-                const float rn = sqrtf(norm2_rn(r));
-                const float rc = rn < 1e-6f ? 1e-6f : rn;
-                const float t = h - rc;
-                const float sg = -spk * (t * t);
-                const float ir = __frcp_rn(rc);
-                const float mj = xj4.w;
-                const float wgt = mj * (sg * ir);
-                const float3 J = make_float3(__fmul_rn(wgt, r.x), __fmul_rn(wgt, r.y), __fmul_rn(wgt, r.z));
-                put_entry(D, row, k, j, J, wgt);
-                rho += mj * cubic_Wq(rn * inv_h, ck);
-                if (j < dyn_end) aii += dot3(J, J) * __frcp_rn(mj);
-                jii = sub3(jii, J);
-            }
-        }
-        const float mi = xi4.w;
-        float dens = 0.0f;
-        dens = dens + mi * P.W0;
-        dens += rho;
-        aii += dot3(jii, jii) * __frcp_rn(mi);
-        const float kd = __frcp_rn(aii + 1e-3f);
-        D.nbr_cnt[row] = n_hit;
-        D.dens[i] = dens;
-        D.kd[i] = kd;
-        D.c[i] = dens - D.rho0s[i];
-        const int pid = D.pid[i];
-        D.rflu[i] = D.material[pid] == 1 ? __frcp_rn(dens) : 0.0f;
-        D.density_out[pid] = dens;
-        D.k_out[pid] = kd;
-        if (found > cap) {
-            atomicAdd(&D.overflow[sc], 1);
-            D.ovf_list[atomicAdd(&D.ovf_ctr[0], 1)] = i;
-            set_cond(D.h_fix, 1u);
-        }
-    }
-    // every row of a slice up to the slice's widest
-    int widest = n_hit;
-    for (int o = 1; o < (32 >> D.lg); o <<= 1) widest = max(widest, __shfl_xor_sync(0xffffffffu, widest, o));
-    if (act) put_pads(D, P.row_base + (i - P.s_begin), n_hit, slice_entries(D, widest), i, 0, 1);
-    // pair count of the scene (a tile never spans scenes): one atomic per CTA
-    int pairs = n_hit;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) pairs += __shfl_xor_sync(0xffffffffu, pairs, o);
-    __shared__ int sh_pairs;
-    if (threadIdx.x == 0) sh_pairs = 0;
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0 && pairs) atomicAdd(&sh_pairs, pairs);
-    __syncthreads();
-    if (threadIdx.x == 0 && sh_pairs) atomicAdd(&D.pairs[sc], (unsigned long long)sh_pairs);
 }
 
 // ---- neighbour-cache overflow: rows of truncated lists and the transpose

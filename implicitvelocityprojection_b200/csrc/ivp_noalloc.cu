@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(32 * kWarps) na_density_aii(int n, Grid g, Scr
         cell = make_int3(cell_coord(xl.x, g.cell_inv, g.dims[0]), cell_coord(xl.y, g.cell_inv, g.dims[1]),
                          cell_coord(xl.z, g.cell_inv, g.dims[2]));
     }
-    const int run = ivp::filter_hits<kSub>(W, B, i0, m, xl, cell, ivp::kHits);
+    const int run = ivp::filter_hits<kSub>(W, B, i0, m, xl, cell, ivp::kHits).run;
     __syncwarp();
     ivp::HitSums s;  // lane p's own particle
     const int found = lane < m ? B.found[lane] : 0;

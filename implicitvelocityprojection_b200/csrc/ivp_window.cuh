@@ -15,14 +15,21 @@ static_assert(kMaxChunks * 32 <= (1 << kOrdShift) && 18 << kOrdShift <= 65536, "
 
 template <int SUB>
 struct BuildShared {
+    static constexpr bool kLists = SUB < 32;           // the hits as lists, or as the ballots' bits
     static constexpr int VMAX = SUB < 16 ? SUB : 16;   // runs with a kept window
-    static constexpr int kRunFill = 3;                 // a run takes in up to two more cells while it holds no more particles
-    float4 pos[SUB];
-    unsigned mask[kMaxChunks][SUB];
+    static constexpr int kRunFill = kLists ? 3 : 12;   // a run takes in up to two more cells while it holds no more particles
+    float4 pos[SUB + 1];                               // (the tests go over particles in pairs)
+    unsigned mask[kMaxChunks][SUB + 1];
     int delta[VMAX][18];                               // slot = delta[run][ordinal] + window position
+    int2 starts[kLists ? 1 : VMAX][kLists ? 1 : kMaxChunks];  // {range starts in the chunk, ordinal before it}
     int found[SUB];                                    // hits of each particle (not capped); -1: scan it alone
-    unsigned short code[kMaxChunks * 32];
-    unsigned short hit[kHits][SUB];
+    unsigned short code[kLists ? kMaxChunks * 32 : 2];
+    unsigned short hit[kLists ? kHits : 1][SUB];
+};
+
+// A lane's particle after the filter pass: its run and the run's chunk count.
+struct RunOf {
+    int run = 0, chunks = 0;
 };
 
 // Largest float r2 with sqrtf(r2) < h: `r2 <= r2_max` is the strict `|r| < h` test
@@ -58,19 +65,23 @@ __device__ __forceinline__ void window_range(const WindowGrid& W, int cx, int cx
 }
 
 // Filter pass of one warp over slots i0 .. i0 + n - 1 (n <= SUB).  Lane l < n
-// passes its particle's position and cell; it returns the lane's run, and leaves
-// every particle's hit count and list in S.
+// passes its particle's position and cell.  With lists, every particle's hit
+// count and list are left in S; without, the ballots of a test with fused
+// products and a slack of 1e-5, which lets a few more through (and the particle
+// itself), for the exact test to come.
 template <int SUB>
-__device__ __forceinline__ int filter_hits(const WindowGrid& W, BuildShared<SUB>& S, int i0, int n, float4 xi,
+__device__ __forceinline__ RunOf filter_hits(const WindowGrid& W, BuildShared<SUB>& S, int i0, int n, float4 xi,
                                              int3 cell, int cap) {
+    constexpr bool LISTS = BuildShared<SUB>::kLists;
     const int lane = threadIdx.x & 31;
     const unsigned le = 0xffffffffu >> (31 - lane);
+    const float r2_near = W.r2_max * 1.00001f;
     if (lane < n) {
         S.pos[lane] = xi;
         S.found[lane] = 0;
     }
     const int row = lane < n ? cell.z * W.dims[1] + cell.y : -1;
-    int mine = 0;
+    RunOf mine;
     __syncwarp();
     for (int first = 0, run = 0; first < n; ++run) {
         const int cx = __shfl_sync(0xffffffffu, cell.x, first);
@@ -111,11 +122,13 @@ __device__ __forceinline__ int filter_hits(const WindowGrid& W, BuildShared<SUB>
             const unsigned rel = (unsigned)(off - 32 * c);
             const unsigned starts = __reduce_or_sync(0xffffffffu, (len > 0 && rel < 32u) ? 1u << rel : 0u);
             const int o = ord + __popc(starts & le);
+            if constexpr (!LISTS)
+                if (lane == 0) S.starts[run][c] = make_int2((int)starts, ord);
             ord += __popc(starts);
             const int v = 32 * c + lane;
             float4 x = make_float4(__int_as_float(0x7fc00000), 0.f, 0.f, 0.f);  // past the end: never within h
             if (v < L) {
-                S.code[v] = (unsigned short)((o << kOrdShift) | v);
+                if constexpr (LISTS) S.code[v] = (unsigned short)((o << kOrdShift) | v);
                 x = __ldg(W.xm + (S.delta[run][o] + v));
             }
             return x;
@@ -125,17 +138,27 @@ __device__ __forceinline__ int filter_hits(const WindowGrid& W, BuildShared<SUB>
         for (int c = 0; c < nch; ++c) {
             const float4 xj = xn;
             if (c + 1 < nch) xn = chunk(c + 1);
-#pragma unroll 4
-            for (int p = 0; p < np; ++p) {
-                const float4 xp = S.pos[first + p];
-                const float3 r = make_float3(xp.x - xj.x, xp.y - xj.y, xp.z - xj.z);
-                const unsigned ball = __ballot_sync(0xffffffffu, norm2_rn(r) <= W.r2_max);
-                if (lane == 0) S.mask[c][first + p] = ball;
+            // two particles at a time; a last odd one tests its successor's
+            // place along, whose ballots its own run writes later
+#pragma unroll 2
+            for (int p = first; p < first + np; p += 2) {
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const float4 xp = S.pos[p + u];
+                    const float3 r = make_float3(xp.x - xj.x, xp.y - xj.y, xp.z - xj.z);
+                    const bool in = LISTS ? norm2_rn(r) <= W.r2_max
+                                          : __fmaf_rn(r.z, r.z, __fmaf_rn(r.y, r.y, r.x * r.x)) <= r2_near;
+                    const unsigned ball = __ballot_sync(0xffffffffu, in);
+                    if (lane == 0) S.mask[c][p + u] = ball;
+                }
             }
         }
         __syncwarp();
-        if (lane >= first && lane < first + np) mine = run;
-        {
+        if (lane >= first && lane < first + np) {
+            mine.run = run;
+            mine.chunks = nch;
+        }
+        if constexpr (LISTS) {
             // expand: lane (c0, p) takes chunks c0, c0 + nc, ... of particle p
             const int sh = np <= 8 ? 3 : np <= 16 ? 4 : 5;
             const int p = lane & ((1 << sh) - 1), c0 = lane >> sh, nc = 32 >> sh;
@@ -177,9 +200,10 @@ struct HitSums {
 };
 
 // The pair terms of hit j at squared distance r2 (sph_kernel.py:8-61) onto the
-// sums; returns J_ij and its weight.
+// sums; returns J_ij, its weight and, where asked, the spline's value.
 __device__ __forceinline__ float3 hit_terms(float3 r, float r2, float mj, bool dynamic, float h, float inv_h,
-                                            float spk, float ck, HitSums& s, float* weight) {
+                                            float spk, float ck, HitSums& s, float* weight,
+                                            float* W = nullptr) {
     // spiky gradient (sph_kernel.py:52-61): -k (h - |r|)^2 r / |r|
     const float rn = sqrtf(r2);
     const float rc = rn < 1e-6f ? 1e-6f : rn;
@@ -188,7 +212,9 @@ __device__ __forceinline__ float3 hit_terms(float3 r, float r2, float mj, bool d
     const float ir = __frcp_rn(rc);
     const float w = mj * (sg * ir);
     const float3 J = make_float3(__fmul_rn(w, r.x), __fmul_rn(w, r.y), __fmul_rn(w, r.z));
-    s.rho += mj * cubic_Wq(rn * inv_h, ck);
+    const float Wr = cubic_Wq(rn * inv_h, ck);
+    s.rho += mj * Wr;
+    if (W) *W = Wr;
     if (dynamic) {
         if (mj != s.m_of) {
             s.m_of = mj;

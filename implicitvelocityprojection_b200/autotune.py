@@ -3,8 +3,7 @@
 The engine's neighbour sums run G lanes per particle in CTAs of G x T
 threads (T particles per tile), either as persistent cooperative solves or as
 one launch per phase, over full {J_ij, j} or compact {j, w_ij} neighbour rows
-(identical bits), after a neighbour build by one thread per particle or one
-warp per cell (identical lists).  Which choice is fastest depends on how many
+(identical bits), after either neighbour build (identical lists).  Which choice is fastest depends on how many
 tiles the scenes make per SM and on their neighbour counts, so the tuner times
 every launch shape on copies of the scenes the caller will run (a few warm-up
 steps, then a few CUDA-event-timed steps each), keeps the fastest, then times
@@ -36,7 +35,7 @@ SHAPES: Tuple[Tuple[int, int], ...] = ((2, 128), (4, 64), (8, 32), (2, 64), (4, 
 # compact {j, w_ij} (8 B, J rebuilt from the positions).  Full rows win while
 # the rows stay in L2; compact rows halve the row stream once they do not.
 ROW_FORMATS: Tuple[int, ...] = (1, 2)
-# neighbour builds with identical lists: one thread per particle, one warp per cell
+# neighbour builds with identical lists: density in list order, by eight lanes
 BUILD_KERNELS: Tuple[int, ...] = (1, 2)
 BUILD_REPS = 5
 

@@ -244,8 +244,8 @@ struct Dev {
     Flags* flags;
     double* err_hist;
     int* pcg_hist;
-    // one scene's statistics gathered for a single device-to-host copy
-    // (StatStage layout)
+    // where k_stage_stats gathers one scene's statistics (StatStage layout;
+    // page-locked host memory)
     unsigned char* stage;
     int hist_len;
     // graph conditionals (0 = not inside a conditional graph)

@@ -103,7 +103,8 @@ struct ivp_engine {
     unsigned long long* h_pairs = nullptr;  // pinned
     double* h_err = nullptr;     // pinned, max_hist: one scene's density-error history
     int* h_pcg = nullptr;        // pinned, max_hist: one scene's CG counts per outer iteration
-    unsigned char* h_stage = nullptr;  // pinned: one scene's statistics block (StatStage)
+    unsigned char* h_stage = nullptr;  // pinned and mapped: one scene's statistics block (StatStage)
+    unsigned char* h_stage_dev = nullptr;  // its device address
 };
 
 // ------------------------------------------------------------ launching
@@ -708,12 +709,11 @@ int run(ivp_engine* e, Emitter emit, cudaGraph_t* g, cudaGraphExec_t* x, cudaStr
 // many tiles per CTA the persistent solves walk fewer, larger tiles per phase
 // (one block reduction per tile); with few, 4 lanes split each row wider.
 constexpr long kAutoTilesPerSM = 16;
-// The thread-per-particle build lasts about one thread's walk of its 27-cell
-// window, so it needs many particles per SM to hide its load latency; below
-// this many dynamic particles per SM the warp-per-cell build (a warp tests a
-// cell's candidates in parallel) is faster (8,192 particles: 0.08 against
-// 0.03 ms; 102,400: 0.117 against 0.129 ms).
-constexpr long kTppMinPerSM = 256;
+// Build kernel 1 (density in list order) costs 2 us more than build kernel 2 up
+// to 31,007 particles (46 and 44 us) and needs 32 particles per warp at 2 lanes
+// per particle, which 262,144 particles repay (197 us; 16 per warp: 215) and
+// few do not (768: 45 and 25 us).
+constexpr long kOrderedMinPerSM = 256;
 
 int resolve_options(const ivp_scene_desc* sc, int n, const ivp_options* in, ivp_options* out) {
     if (!in || !out) return IVP_ERR_BAD_ARG;
@@ -733,7 +733,7 @@ int resolve_options(const ivp_scene_desc* sc, int n, const ivp_options* in, ivp_
             sms = 148;
         }
         if (in->lanes_per_particle == 0) out->lanes_per_particle = tiles > kAutoTilesPerSM * sms ? 2 : 4;
-        if (in->build_kernel == 0) out->build_kernel = dyn >= kTppMinPerSM * sms ? 1 : 2;
+        if (in->build_kernel == 0) out->build_kernel = dyn >= kOrderedMinPerSM * sms ? 1 : 2;
     }
     if (in->particles_per_block == 0 && out->lanes_per_particle > 0)
         out->particles_per_block = 256 / out->lanes_per_particle;
@@ -944,8 +944,7 @@ void plan(const ivp_scene_desc* sc, int n, const ivp_options* o, Plan& P) {
     P.off[i++] = L.add(sizeof(float4) * N);                                    // 62 vpp
     P.off[i++] = L.add(sizeof(float4) * N);                                    // 63 vlp
     P.off[i++] = L.add(P.any_st ? sizeof(float4) * N : 0);                     // 64 stz
-    P.off[i++] = L.add(StatStage(o->max_hist).total);                          // 65 stage
-    P.off[i++] = L.add(sizeof(float) * N);                                     // 66 jd
+    P.off[i++] = L.add(sizeof(float) * N);                                     // 65 jd
 }
 
 cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
@@ -954,13 +953,15 @@ cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 // mirrors are enqueued on the caller's stream, the caller synchronises once,
 // then the fill functions convert.
 // One scene's statistics and histories (the whole history rows, max_hist
-// entries each) in one device-to-host copy after a gather kernel, instead of
-// one copy per array; unpack_stage places them in the host mirrors.
+// entries each): a gather kernel writes them straight into the page-locked
+// staging block (2 KB over the bus; a copy behind the kernel took another 6 us
+// of every statistics read); unpack_stage places them in the host mirrors.
 int enqueue_stage(ivp_engine* e, int scene, cudaStream_t s) {
     const int H = e->opt.max_hist;
-    k_stage_stats<<<1, 256, 0, s>>>(e->D, scene, H);
+    Dev D = e->D;
+    D.stage = e->h_stage_dev;
+    k_stage_stats<<<1, 256, 0, s>>>(D, scene, H);
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(e->h_stage, e->D.stage, StatStage(H).total, cudaMemcpyDeviceToHost, s));
     return IVP_OK;
 }
 
@@ -1163,7 +1164,6 @@ int ivp_engine_create(const ivp_scene_desc* scenes, int32_t n_scenes, const ivp_
     D.vpp = reinterpret_cast<float4*>(w + P.off[i++]);
     D.vlp = reinterpret_cast<float4*>(w + P.off[i++]);
     D.stz = reinterpret_cast<float4*>(w + P.off[i++]);
-    D.stage = reinterpret_cast<unsigned char*>(w + P.off[i++]);
     D.jd = reinterpret_cast<float*>(w + P.off[i++]);
     D.drop_cap = P.drop_cap;
     e->fix_scan_blocks = P.fix_scan_blocks;
@@ -1218,7 +1218,8 @@ int ivp_engine_create(const ivp_scene_desc* scenes, int32_t n_scenes, const ivp_
         cudaHostAlloc((void**)&e->h_pcg, sizeof(int) * opt->max_hist, cudaHostAllocDefault) != cudaSuccess ||
         cudaHostAlloc((void**)&e->h_ovf, sizeof(int), cudaHostAllocDefault) != cudaSuccess ||
         cudaHostAlloc((void**)&e->h_fix_scene, sizeof(int) * n_scenes, cudaHostAllocDefault) != cudaSuccess ||
-        cudaHostAlloc((void**)&e->h_stage, StatStage(opt->max_hist).total, cudaHostAllocDefault) != cudaSuccess)
+        cudaHostAlloc((void**)&e->h_stage, StatStage(opt->max_hist).total, cudaHostAllocMapped) != cudaSuccess ||
+        cudaHostGetDevicePointer((void**)&e->h_stage_dev, e->h_stage, 0) != cudaSuccess)
         return fail(IVP_ERR_CUDA);
     if (cudaMemcpyAsync((void*)D.scenes, P.hp.data(), sizeof(SceneParams) * n_scenes, cudaMemcpyHostToDevice, s) !=
             cudaSuccess ||

@@ -2364,9 +2364,8 @@ __device__ bool grid_all_reduce_barrier(const Dev& D, int kind, const double* pa
         volatile unsigned* cnt = D.bar_count;
         int ok = 1;
         const unsigned long long t0 = globaltimer_ns();
-        while ((int)(*cnt - target) < 0) {
-            __nanosleep(32);
-            if (globaltimer_ns() - t0 > D.bar_limit_ns) {
+        for (unsigned n = 0; (int)(*cnt - target) < 0; ++n) {
+            if ((n & 15u) == 0u && globaltimer_ns() - t0 > D.bar_limit_ns) {
                 ok = 0;
                 D.flags->timeout = 1;
                 break;
@@ -2407,9 +2406,9 @@ __device__ bool grid_reduce_barrier(const Dev& D, int kind, const double* partia
         // before arriving) is the current one
         volatile unsigned* gen = D.bar_gen;
         const unsigned long long t0 = globaltimer_ns();
-        while (*gen == g) {
+        for (unsigned n = 0; *gen == g; ++n) {
             __nanosleep(32);
-            if (globaltimer_ns() - t0 > D.bar_limit_ns) {
+            if ((n & 15u) == 0u && globaltimer_ns() - t0 > D.bar_limit_ns) {
                 sh_flag[1] = 0;
                 D.flags->timeout = 1;
                 break;
@@ -2580,7 +2579,7 @@ struct Phaser {
         auto& wt_sh = S.tile;
         const int wid = threadIdx.x >> 5, wl = threadIdx.x & 31;
         int nb = 0;
-        auto flush = [&]() {
+        auto flush = [&](bool last) {
             __syncthreads();
             double* pb = partials();
             for (int s = wid; s < nb; s += NW) {
@@ -2596,7 +2595,7 @@ struct Phaser {
                     if (kind == K_V_B) pb[D.n_tiles + wt_sh[s]] = t2;
                 }
             }
-            __syncthreads();
+            if (!last) __syncthreads();  // (the grid barrier starts with one)
             nb = 0;
         };
         int sc = (int)blockIdx.x < A ? scene_of(blockIdx.x) : 0;
@@ -2655,9 +2654,9 @@ struct Phaser {
                 ws_sh[1][nb][wid] = w2;
             }
             if (threadIdx.x == 0) wt_sh[nb] = t;
-            if (++nb == kFlushTiles) flush();
+            if (++nb == kFlushTiles) flush(false);
         }
-        if (nb) flush();  // nb is the same in every thread
+        if (nb) flush(true);  // nb is the same in every thread
         if (!barrier((kind == K_ST_DIV || kind == K_PJ_HEAD) ? -1 : kind)) return false;
         if (++phases > D.phase_limit) {
             // guard: every CTA reaches the same count; CTA 0 stops the scenes,

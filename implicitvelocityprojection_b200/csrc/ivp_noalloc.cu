@@ -113,8 +113,9 @@ __global__ void na_order(const float* __restrict__ x, const float* __restrict__ 
 //
 // One warp per eight slots, as in the engine's build for small scenes: a thread
 // per particle walked 270 candidates one after another, on 176 CTAs of 256
-// threads for 40,000 particles (99 us), and left most of the chip waiting.
-constexpr int kSub = 8, kWarps = 2;
+// threads for 40,000 particles (99 us), and left most of the chip waiting.  One warp per CTA: 60 us a call;
+// two: 63 to 73.
+constexpr int kSub = 8, kWarps = 1;
 
 __global__ void __launch_bounds__(32 * kWarps) na_density_aii(int n, Grid g, Scratch* S, float* __restrict__ density,
                                                               float* __restrict__ kdiag) {

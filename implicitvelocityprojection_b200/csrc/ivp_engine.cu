@@ -371,7 +371,7 @@ int emit_build_impl(ivp_engine* e, Launcher& L, bool with_advect) {
             CK(cudaGraphConditionalHandleCreate(&h_fix, L.graph, 0, cudaGraphCondAssignDefault));
             copy.h_fix = (unsigned long long)h_fix;
         }
-        // Build kernel 1 sums the density in list order: eight slots a warp at
+        // Build kernel 1 sums density and k in list order: eight slots a warp at
         // 4 and 8 lanes per particle, 32 at 1 and 2 (many particles: fewer
         // windows walked).  Build kernel 2 does not; its warps take eight slots
         // or a slice of rows.  A warp never takes less than a slice, whose rows
@@ -709,10 +709,11 @@ int run(ivp_engine* e, Emitter emit, cudaGraph_t* g, cudaGraphExec_t* x, cudaStr
 // many tiles per CTA the persistent solves walk fewer, larger tiles per phase
 // (one block reduction per tile); with few, 4 lanes split each row wider.
 constexpr long kAutoTilesPerSM = 16;
-// Build kernel 1 (density in list order) costs 2 us more than build kernel 2 up
-// to 31,007 particles (46 and 44 us) and needs 32 particles per warp at 2 lanes
-// per particle, which 262,144 particles repay (197 us; 16 per warp: 215) and
-// few do not (768: 45 and 25 us).
+// Build kernel 1 adds density, Aii and J_ii in list order, build kernel 2 by eight
+// lanes; the line keeps each size's sums what one thread per particle and one warp
+// per cell made them.  Kernel 1 costs 3 us more for 768 particles (26 and 23 us),
+// 5 for 31,007 (42 and 38), 18 for 262,144 at 2 lanes per particle (198 and 180)
+// and is 6 faster for 524,288 (333 and 339).
 constexpr long kOrderedMinPerSM = 256;
 
 int resolve_options(const ivp_scene_desc* sc, int n, const ivp_options* in, ivp_options* out) {

@@ -465,18 +465,35 @@ __global__ void k_order(const Dev D) {
 //   SUB = 8, or a slice of rows where that is more: the bits are expanded into
 //   hit lists and eight lanes share a particle; more warps with shorter chains
 //   of loads.
-// ORDERED adds the density in list order, as the reference does (SUB = 32 does by
-// its nature): rho - rho0 cancels all but the last digits of the sum, and a
+// ORDERED adds density, Aii and J_ii in list order, as the reference does (SUB = 32
+// does by its nature): rho - rho0 cancels all but the last digits of the sum, and a
 // constraint near zero falls on one side of the operator's switch or the other.
+// Lanes that share a particle then pass their hits' factors through shared memory
+// to one chain per sum (ListOrder).  At 4 lanes per particle: 98 us for 102,400
+// particles (87 by eight lanes), 69 (62) for 60,000, 26 (23) for 768.
 constexpr int kBuildWarps = 1;  // warps per CTA: they share nothing, and a CTA's slot is free as soon as its warp is done
 
-// All hits of one particle by the whole warp, straight from its window: for
-// windows that do not fit the filter pass.  Every lane returns the sums;
-// `entry(k, j, J, w)` is called by the lane of each kept hit.
-template <class Entry>
-__device__ __forceinline__ int scan_alone(const WindowGrid& W, int* list, int i, float4 xi, int3 cell, int cap,
-                                          int dyn_end, float h, float inv_h, float spk, float ck, HitSums& s,
-                                          Entry&& entry) {
+// N lanes (8 or 32) sum the n_hit hits of a particle in list order: `take(k, a, W,
+// jj, J)` computes hit k and returns m_j.  n_hit is the same in the N lanes; the
+// whole warp calls it.
+template <int N, class Take>
+__device__ __forceinline__ void sum_in_list_order(int n_hit, float* mem, HitSums& a, Take&& take) {
+    const int lane = threadIdx.x & 31;
+    ListOrder<N> order;
+    for (int k0 = 0; k0 < n_hit; k0 += N) {
+        const int k = k0 + (lane & (N - 1));
+        float mj = 0.0f, W = 0.0f, jj = 0.0f;
+        float3 J = make_float3(0.0f, 0.0f, 0.0f);
+        if (k < n_hit) mj = take(k, a, &W, &jj, &J);
+        order.add(mem, N == 32 ? 0xffffffffu : ((1u << N) - 1u) << (lane & (32 - N)), mj, W, jj, a.inv_m, J);
+    }
+    __syncwarp();
+    order.get(a);
+}
+
+// The hits of one particle by the whole warp, straight from its window: for
+// windows that do not fit the filter pass.  The first `cap` go to `list`.
+__device__ __forceinline__ int scan_alone(const WindowGrid& W, int* list, int i, float4 xi, int3 cell, int cap) {
     const int lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1u;
     int b, len;
@@ -497,17 +514,6 @@ __device__ __forceinline__ int scan_alone(const WindowGrid& W, int* list, int i,
             found += __popc(ball);
         }
     }
-    __syncwarp();
-    const int n_hit = min(found, cap);
-    for (int k = lane; k < n_hit; k += 32) {
-        const int j = list[k];
-        const float4 xj = __ldg(W.xm + j);
-        const float3 r = make_float3(xi.x - xj.x, xi.y - xj.y, xi.z - xj.z);
-        float w;
-        const float3 J = hit_terms(r, norm2_rn(r), xj.w, j < dyn_end, h, inv_h, spk, ck, s, &w);
-        entry(k, j, J, w);
-    }
-    sum_lanes<32>(s);
     __syncwarp();
     return found;
 }
@@ -556,12 +562,19 @@ __global__ void __launch_bounds__(32 * kBuildWarps) k_nbr_build(const Dev D, int
     }
     const RunOf mine = filter_hits<SUB>(W, S, i0, n, xl, cell, cap);
     __syncwarp();
-    // the row entry, density and Aii terms of hit k of slot i
-    auto take = [&](int i, int k, int j, float4 xi, float4 xj, float3 r, float r2, HitSums& s) {
-        float w, Wj;
-        const float3 J = hit_terms(r, r2, xj.w, j < dyn_end, h, inv_h, spk, ck, s, &w, &Wj);
+    // the row entry, density and Aii terms of hit k (slot j) of slot i
+    auto take = [&](int i, int k, int j, float4 xi, float4 xj, float3 r, float r2, HitSums& s, float* Wj = nullptr,
+                    float* jj = nullptr) {
+        float w;
+        const float3 J = hit_terms(r, r2, xj.w, j < dyn_end, h, inv_h, spk, ck, s, &w, Wj, jj);
         put_entry(D, P.row_base + (i - P.s_begin), k, j, J, w);
-        return Wj;
+        return J;
+    };
+    auto take_slot = [&](int i, int k, int j, float4 xi, HitSums& s, float* Wj, float* jj, float3* J) {
+        const float4 xj = __ldg(D.xm + j);
+        const float3 r = make_float3(xi.x - xj.x, xi.y - xj.y, xi.z - xj.z);
+        *J = take(i, k, j, xi, xj, r, norm2_rn(r), s, Wj, jj);
+        return xj.w;
     };
     HitSums s;      // lane p's own particle
     int found = lane < n ? S.found[lane] : 0;
@@ -602,8 +615,25 @@ __global__ void __launch_bounds__(32 * kBuildWarps) k_nbr_build(const Dev D, int
                 }
             }
         }
-    } else {
-        // eight lanes per particle, four particles at a time
+        __syncwarp();
+        // particles scanned alone, by the whole warp (the ballots have been used)
+        int* list = reinterpret_cast<int*>(S.mask);
+        static_assert(sizeof(S.mask) >= (kHits + ListOrder<32>::kWords) * sizeof(float));
+        for (unsigned left = alone; left; left &= left - 1u) {
+            const int q = __ffs(left) - 1;
+            const float4 xq = S.pos[q];
+            const int f = scan_alone(W, list, i0 + q, xq, cell_of(xq), cap);
+            HitSums a;
+            sum_in_list_order<32>(min(f, cap), reinterpret_cast<float*>(list) + kHits, a,
+                                  [&](int k, HitSums& t, float* Wj, float* jj, float3* J) {
+                                      return take_slot(i0 + q, k, list[k], xq, t, Wj, jj, J);
+                                  });
+            if (lane == q) {
+                s = a;
+                found = f;
+            }
+        }
+    } else if constexpr (!ORDERED) {
         const int sub = lane & 7;
         for (int p0 = 0; p0 < n; p0 += 4) {
             const int p = p0 + (lane >> 3);
@@ -611,44 +641,81 @@ __global__ void __launch_bounds__(32 * kBuildWarps) k_nbr_build(const Dev D, int
             const int* delta = S.delta[__shfl_sync(0xffffffffu, mine.run, min(p, n - 1))];
             const float4 xi = S.pos[min(p, n - 1)];
             HitSums a;
-            float rho = 0.0f;
             for (int k0 = 0; k0 < n_hit; k0 += 8) {  // the same in a particle's lanes
                 const int k = k0 + sub;
-                float mj = 0.0f, Wj = 0.0f;
                 if (k < n_hit) {
                     const int code = S.hit[k][p];
                     const int j = delta[code >> kOrdShift] + (code & ((1 << kOrdShift) - 1));
                     const float4 xj = __ldg(D.xm + j);
                     const float3 r = make_float3(xi.x - xj.x, xi.y - xj.y, xi.z - xj.z);
-                    Wj = take(i0 + p, k, j, xi, xj, r, norm2_rn(r), a);
-                    mj = xj.w;
-                }
-                if constexpr (ORDERED) {
-                    const unsigned group = 0xffu << (lane & 24);
-#pragma unroll
-                    for (int q = 0; q < 8; ++q)
-                        rho = __fmaf_rn(__shfl_sync(group, mj, (lane & 24) + q), __shfl_sync(group, Wj, (lane & 24) + q), rho);
+                    take(i0 + p, k, j, xi, xj, r, norm2_rn(r), a);
                 }
             }
             __syncwarp();
             sum_lanes<8>(a);
-            if constexpr (ORDERED) a.rho = rho;
-            own_sums(a, p0, s);
+            own_sums(a, p0, 4, s);
+        }
+        __syncwarp();
+        // particles scanned alone (their list takes the ballots' place): the sums of
+        // eight lanes, as above; the other lanes repeat them, which costs less code
+        int* list = reinterpret_cast<int*>(S.mask);
+        for (unsigned left = alone; left; left &= left - 1u) {
+            const int q = __ffs(left) - 1;
+            const float4 xq = S.pos[q];
+            const int f = scan_alone(W, list, i0 + q, xq, cell_of(xq), cap);
+            HitSums a;
+            const int nh = min(f, cap);
+            for (int k = lane & 7; k < nh; k += 8) {
+                const int j = list[k];
+                const float4 xj = __ldg(D.xm + j);
+                const float3 r = make_float3(xq.x - xj.x, xq.y - xj.y, xq.z - xj.z);
+                take(i0 + q, k, j, xq, xj, r, norm2_rn(r), a);
+            }
+            __syncwarp();
+            sum_lanes<8>(a);
+            if (lane == q) {
+                s = a;
+                found = f;
+            }
+        }
+    } else {
+        // the same in list order, in one loop
+        static_assert(sizeof(S.code) >= 4 * ListOrder<8>::kWords * sizeof(float));
+        float* mem = reinterpret_cast<float*>(S.code) + ListOrder<8>::kWords * (lane >> 3);  // (read last by the filter)
+        int* list = reinterpret_cast<int*>(S.mask);
+        unsigned left = alone;
+        for (int p0 = 0, count = 4; p0 < n || left; p0 += 4) {
+            int p = p0 + (lane >> 3), n_hit;
+            const int* delta = nullptr;
+            if (p0 < n) {
+                n_hit = p < n ? min(S.found[p], cap) : 0;
+                delta = S.delta[__shfl_sync(0xffffffffu, mine.run, min(p, n - 1))];
+                p = min(p, n - 1);
+            } else {
+                p = __ffs(left) - 1;
+                left &= left - 1u;
+                const float4 xp = S.pos[p];
+                const int f = scan_alone(W, list, i0 + p, xp, cell_of(xp), cap);
+                if (lane == p) found = f;
+                n_hit = lane < 8 ? min(f, cap) : 0;
+                count = 1;
+            }
+            const float4 xi = S.pos[p];
+            HitSums a;
+            sum_in_list_order<8>(n_hit, mem, a, [&](int k, HitSums& t, float* Wj, float* jj, float3* J) {
+                int j;
+                if (delta) {
+                    const int code = S.hit[k][p];
+                    j = delta[code >> kOrdShift] + (code & ((1 << kOrdShift) - 1));
+                } else {
+                    j = list[k];
+                }
+                return take_slot(i0 + p, k, j, xi, t, Wj, jj, J);
+            });
+            own_sums(a, count == 4 ? p0 : p, count, s);
         }
     }
     __syncwarp();
-    for (unsigned left = alone; left; left &= left - 1u) {
-        const int q = __ffs(left) - 1;
-        const float4 xq = S.pos[q];
-        const int rq = P.row_base + (i0 + q - P.s_begin);
-        HitSums a;
-        const int f = scan_alone(W, reinterpret_cast<int*>(S.mask), i0 + q, xq, cell_of(xq), cap, dyn_end, h, inv_h,
-                                 spk, ck, a, [&](int k, int j, float3 J, float w) { put_entry(D, rq, k, j, J, w); });
-        if (lane == q) {
-            s = a;
-            found = f;
-        }
-    }
     // every row of a slice up to the slice's widest
     const bool act = lane < n;
     const int i = i0 + (act ? lane : 0), row = P.row_base + (i - P.s_begin);
@@ -661,7 +728,7 @@ __global__ void __launch_bounds__(32 * kBuildWarps) k_nbr_build(const Dev D, int
         float dens = 0.0f;
         dens = dens + mi * P.W0;
         dens += s.rho;
-        const float aii = s.aii + dot3(s.jii, s.jii) * __frcp_rn(mi);
+        const float aii = __fmaf_rn(length2(s.jii), __frcp_rn(mi), s.aii);
         const float kd = __frcp_rn(aii + 1e-3f);
         D.nbr_cnt[row] = pairs;
         D.dens[i] = dens;

@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(32 * kWarps) na_density_aii(int n, Grid g, Scr
         }
         __syncwarp();
         ivp::sum_lanes<8>(a);
-        ivp::own_sums(a, p0, s);
+        ivp::own_sums(a, p0, 4, s);
     }
     for (unsigned left = alone; left; left &= left - 1u) {
         const int p = __ffs(left) - 1, i = i0 + p;

@@ -23,7 +23,7 @@ struct BuildShared {
     int delta[VMAX][18];                               // slot = delta[run][ordinal] + window position
     int2 starts[kLists ? 1 : VMAX][kLists ? 1 : kMaxChunks];  // {range starts in the chunk, ordinal before it}
     int found[SUB];                                    // hits of each particle (not capped); -1: scan it alone
-    unsigned short code[kLists ? kMaxChunks * 32 : 2];
+    alignas(16) unsigned short code[kLists ? kMaxChunks * 32 : 2];
     unsigned short hit[kLists ? kHits : 1][SUB];
 };
 
@@ -199,11 +199,19 @@ struct HitSums {
     float3 jii = make_float3(0.0f, 0.0f, 0.0f);
 };
 
+// |a|^2, its roundings written out: left to the compiler, the product that stays
+// outside the fused steps differed between two kernels, and with it the last bit
+// of k.
+__device__ __forceinline__ float length2(float3 a) {
+    return __fmaf_rn(a.z, a.z, __fmaf_rn(a.x, a.x, __fmul_rn(a.y, a.y)));
+}
+
 // The pair terms of hit j at squared distance r2 (sph_kernel.py:8-61) onto the
-// sums; returns J_ij, its weight and, where asked, the spline's value.
+// sums; returns J_ij, its weight and, where asked, the spline's value and the
+// squared length of a dynamic neighbour's J_ij (its 1 / m is then s.inv_m).
 __device__ __forceinline__ float3 hit_terms(float3 r, float r2, float mj, bool dynamic, float h, float inv_h,
                                             float spk, float ck, HitSums& s, float* weight,
-                                            float* W = nullptr) {
+                                            float* W = nullptr, float* JJ = nullptr) {
     // spiky gradient (sph_kernel.py:52-61): -k (h - |r|)^2 r / |r|
     const float rn = sqrtf(r2);
     const float rc = rn < 1e-6f ? 1e-6f : rn;
@@ -213,14 +221,16 @@ __device__ __forceinline__ float3 hit_terms(float3 r, float r2, float mj, bool d
     const float w = mj * (sg * ir);
     const float3 J = make_float3(__fmul_rn(w, r.x), __fmul_rn(w, r.y), __fmul_rn(w, r.z));
     const float Wr = cubic_Wq(rn * inv_h, ck);
-    s.rho += mj * Wr;
+    s.rho = __fmaf_rn(mj, Wr, s.rho);
     if (W) *W = Wr;
     if (dynamic) {
         if (mj != s.m_of) {
             s.m_of = mj;
             s.inv_m = __frcp_rn(mj);
         }
-        s.aii += dot3(J, J) * s.inv_m;
+        const float jj = length2(J);
+        s.aii = __fmaf_rn(jj, s.inv_m, s.aii);
+        if (JJ) *JJ = jj;
     }
     s.jii = sub3(s.jii, J);
     *weight = w;
@@ -239,17 +249,71 @@ __device__ __forceinline__ void sum_lanes(HitSums& s) {
     }
 }
 
-// The sums of particles p0 .. p0 + 3, in the eight lanes of each, to the lanes
-// p0 .. p0 + 3.
-__device__ __forceinline__ void own_sums(const HitSums& a, int p0, HitSums& s) {
-    const int lane = threadIdx.x & 31, from = ((lane - p0) * 8) & 31;
+// The sums that lane `from` holds.
+__device__ __forceinline__ HitSums sums_of_lane(const HitSums& a, int from) {
     HitSums g;
     g.rho = __shfl_sync(0xffffffffu, a.rho, from);
     g.aii = __shfl_sync(0xffffffffu, a.aii, from);
     g.jii.x = __shfl_sync(0xffffffffu, a.jii.x, from);
     g.jii.y = __shfl_sync(0xffffffffu, a.jii.y, from);
     g.jii.z = __shfl_sync(0xffffffffu, a.jii.z, from);
-    if (lane >= p0 && lane < p0 + 4) s = g;
+    return g;
 }
+
+// The sums of particles p0 .. p0 + count - 1 (count <= 4), in the eight lanes of
+// each, to the lanes p0 .. p0 + count - 1.
+__device__ __forceinline__ void own_sums(const HitSums& a, int p0, int count, HitSums& s) {
+    const int lane = threadIdx.x & 31;
+    const HitSums g = sums_of_lane(a, ((lane - p0) * 8) & 31);
+    if (lane >= p0 && lane < p0 + count) s = g;
+}
+
+// Sums in list order by N lanes, one hit each: five sums (rho, Aii, J_ii), each a
+// chain of fma(first, second, sum) over the hits.  The lanes leave their hits'
+// factors in shared memory and lane q < 5 of the N runs the chain of sum q.
+template <int N>
+struct ListOrder {
+    static constexpr int kWords = 7 * N;  // m_j, W, |J|^2, 1 / m_j, J of N hits
+    float sum = 0.0f;
+
+    // Factors of zero add nothing; `group` is the mask of the N lanes, `mem` their
+    // kWords words (16-byte aligned).
+    __device__ __forceinline__ void add(float* mem, unsigned group, float mj, float W, float jj, float inv_m,
+                                        float3 J) {
+        const int sub = threadIdx.x & (N - 1);
+        mem[sub] = mj;
+        mem[N + sub] = W;
+        mem[2 * N + sub] = jj;
+        mem[3 * N + sub] = inv_m;
+        mem[4 * N + sub] = J.x;
+        mem[5 * N + sub] = J.y;
+        mem[6 * N + sub] = J.z;
+        __syncwarp(group);
+        const int q = min(sub, 4);
+        const float4* first = reinterpret_cast<const float4*>(mem + N * (q < 2 ? 2 * q : 2 + q));
+        const float4* second = reinterpret_cast<const float4*>(mem + N * (q < 2 ? 2 * q + 1 : 0));
+#pragma unroll 2
+        for (int u = 0; u < N / 4; ++u) {
+            const float4 a = first[u];
+            float4 b = second[u];
+            if (q >= 2) b = make_float4(-1.0f, -1.0f, -1.0f, -1.0f);
+            sum = __fmaf_rn(a.x, b.x, sum);
+            sum = __fmaf_rn(a.y, b.y, sum);
+            sum = __fmaf_rn(a.z, b.z, sum);
+            sum = __fmaf_rn(a.w, b.w, sum);
+        }
+        __syncwarp(group);
+    }
+
+    // The five sums in every lane of the N (the whole warp calls it).
+    __device__ __forceinline__ void get(HitSums& s) const {
+        const int g = threadIdx.x & (32 - N);
+        s.rho = __shfl_sync(0xffffffffu, sum, g);
+        s.aii = __shfl_sync(0xffffffffu, sum, g + 1);
+        s.jii.x = __shfl_sync(0xffffffffu, sum, g + 2);
+        s.jii.y = __shfl_sync(0xffffffffu, sum, g + 3);
+        s.jii.z = __shfl_sync(0xffffffffu, sum, g + 4);
+    }
+};
 
 }  // namespace ivp

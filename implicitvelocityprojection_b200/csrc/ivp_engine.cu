@@ -242,8 +242,11 @@ struct Launcher {
 struct KernelSet {
     DevKernel pack, rhs, cg_a, cg_b, dens, aii, div, v_setup, v_a, v_b, v_end, st_div, pj_head, pj_tail;
     DevKernel persist, v_persist, st_persist, prj_persist;  // for the engine's row format
-    size_t persist_smem;
+    size_t persist_smem, persist_smem_max;           // of this engine, of any engine
 };
+
+// Scenes of an engine that runs the persistent solves.
+constexpr int kPersistScenes = 256;
 
 template <int G, int B, int F>
 void set_persistent(KernelSet& K, int n_scenes) {
@@ -252,6 +255,7 @@ void set_persistent(KernelSet& K, int n_scenes) {
     K.st_persist = k_force_persistent<G, B, F, FORCE_ST>;
     K.prj_persist = k_prj_persistent<G, B, F>;
     K.persist_smem = Phaser<G, B, F>::shared_bytes(n_scenes);
+    K.persist_smem_max = std::max(Phaser<G, B, F>::shared_bytes(kParamScenes), Phaser<G, B, F>::shared_bytes(kPersistScenes));
 }
 
 template <int G, int B>
@@ -267,6 +271,18 @@ KernelSet make_set(int read, int n_scenes) {
 
 int row_read(const Dev& D) {
     return D.row_fmt != ROW_FULL ? READ_ANY : D.row_stream ? READ_STREAM : READ_FULL;
+}
+
+// Lets a kernel be launched with the engine's dynamic shared memory.  The limit
+// belongs to the kernel and so to every engine of the process: it is only ever
+// raised, and then to what the largest engine needs, which leaves nothing to the
+// order in which engines are created.
+bool allow_shared(DevKernel k, const KernelSet& K) {
+    cudaFuncAttributes a;
+    if (cudaFuncGetAttributes(&a, (const void*)k) != cudaSuccess) return false;
+    if (K.persist_smem <= (size_t)a.maxDynamicSharedSizeBytes) return true;
+    return cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)K.persist_smem_max) == cudaSuccess;
 }
 
 // Instantiated launch shapes: G lanes per particle x {128, 256} threads.
@@ -1233,16 +1249,14 @@ int ivp_engine_create(const ivp_scene_desc* scenes, int32_t n_scenes, const ivp_
     if (cudaStreamSynchronize(s) != cudaSuccess) return fail(IVP_ERR_CUDA);
     // persistent solve: a co-resident grid of at most one CTA per tile
     e->persistent = false;
-    if (opt->persistent && e->n_tiles > 0 && n_scenes <= 256) {
+    if (opt->persistent && e->n_tiles > 0 && n_scenes <= kPersistScenes) {
         int dev = 0, coop = 0, nsm = 0, per_sm = 0;
         KernelSet K;
         kernel_set(e->G, e->BLOCK, row_read(e->D), e->n_scenes, &K);
         e->coop_smem = K.persist_smem;
-        for (DevKernel k : {K.persist, K.v_persist, K.st_persist, K.prj_persist})
-            if (cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e->coop_smem) !=
-                cudaSuccess)
-                return fail(IVP_ERR_CUDA);
-        if (cudaGetDevice(&dev) == cudaSuccess &&
+        bool fits = true;
+        for (DevKernel k : {K.persist, K.v_persist, K.st_persist, K.prj_persist}) fits = fits && allow_shared(k, K);
+        if (fits && cudaGetDevice(&dev) == cudaSuccess &&
             cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) == cudaSuccess && coop &&
             cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)K.persist, e->BLOCK, e->coop_smem) ==
@@ -1263,6 +1277,7 @@ int ivp_engine_create(const ivp_scene_desc* scenes, int32_t n_scenes, const ivp_
                 e->persistent = true;
             }
         }
+        cudaGetLastError();  // an engine without persistent solves is a working engine
     }
     *out = e;
     return IVP_OK;

@@ -1,0 +1,41 @@
+"""Several engines in one process: what one engine sets up on the kernels that
+they share holds for the others, in whatever order engines are created and used."""
+import numpy as np
+import pytest
+
+import _gpu_helpers as H
+from implicitvelocityprojection_b200 import scenes as S
+
+pytestmark = pytest.mark.gpu
+
+
+def _scenes(n, first=0):
+    return [S.random_column(400 + 60 * k, 2.0, seed=200 + first + k, viscosity_method=1, viscosity_coeff=1e-3)
+            for k in range(n)]
+
+
+def _solve(eng, n):
+    """A force on its own, then a step: direct launches and (with graphs) a graph
+    that is built at this first use."""
+    eng.build()
+    eng.viscosity_solve()
+    eng.step(1)
+    assert all(eng.stats(i).status == 0 for i in range(n))
+    return [np.concatenate([eng.get("x", i), eng.get("v", i)]) for i in range(n)]
+
+
+@pytest.mark.parametrize("use_graphs", [True, False])
+@pytest.mark.parametrize("n,others", [(3, (1,)), (4, (5,)), (8, (1, 3)), (256, (1,))])
+def test_engines_created_later_leave_earlier_ones_working(n, others, use_graphs):
+    """The persistent kernels' shared memory grows with the engine's scenes (and
+    four scenes take more than five, whose parameters stay in global memory; 256
+    take more than the 48 KB that a kernel may use without asking).  Engines of
+    other sizes, created in between and used first, change nothing."""
+    scs = _scenes(n)
+    alone = _solve(H.engine(scs, use_graphs=use_graphs), n)
+    eng = H.engine(scs, use_graphs=use_graphs)
+    later = [H.engine(_scenes(k, 500), use_graphs=use_graphs) for k in others]
+    for k, e in zip(others, later):
+        _solve(e, k)
+    for a, b in zip(alone, _solve(eng, n)):
+        assert np.array_equal(a, b)

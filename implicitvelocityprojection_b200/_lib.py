@@ -138,6 +138,7 @@ SIGNATURES = {
                             ctypes.POINTER(_I)]),
     "ivp_export_neighbours": (_I, [_P, _I, _P, _P, _I, _P]),
     "ivp_set_wait_limit": (_I, [_P, ctypes.c_int64]),
+    "ivp_fail_launch": (_I, [_P, _I]),
     "ivp_prepare": (_I, [_P]),
     "ivp_read_stats_all": (_I, [_P, _P, ctypes.POINTER(SolveStats)]),
     "ivp_density_aii_noalloc": (_I, [_P, _P, _P, _I, ctypes.c_float, _P, _I, _P, _P, _P]),

@@ -105,6 +105,7 @@ struct ivp_engine {
     int* h_pcg = nullptr;        // pinned, max_hist: one scene's CG counts per outer iteration
     unsigned char* h_stage = nullptr;  // pinned and mapped: one scene's statistics block (StatStage)
     unsigned char* h_stage_dev = nullptr;  // its device address
+    int fail_in = 0;             // test hook: launches until one fails (0: none does)
 };
 
 // ------------------------------------------------------------ launching
@@ -129,6 +130,7 @@ struct Launcher {
     cudaGraphNode_t last = nullptr;
     bool has_last = false;
     Prof* prof = nullptr;
+    int* fail_in = nullptr;          // ivp_engine::fail_in (launches on a stream)
     // host copies of an ivp_step_io step (null otherwise), and a node the
     // next chained node must also wait for (graph mode)
     ivp_engine* io = nullptr;
@@ -154,6 +156,10 @@ struct Launcher {
     int kernel(int id, const void* fn, dim3 grid, dim3 block, void** args, size_t smem = 0, bool coop = false) {
         if (grid.x == 0) return IVP_OK;
         if (!graph) {
+            if (fail_in && *fail_in > 0 && --*fail_in == 0) {
+                g_err = "launch stopped by ivp_fail_launch";
+                return IVP_ERR_CUDA;
+            }
             if (prof) {
                 const size_t k = prof->ids.size();
                 while (prof->ev.size() < 2 * (k + 1)) {
@@ -708,6 +714,22 @@ int make_graph(ivp_engine* e, Emitter emit, cudaGraph_t* g, cudaGraphExec_t* x) 
     return IVP_OK;
 }
 
+// A call's launches on a stream.  Where they stop half-way, the barrier counters
+// that a solve before left nonzero are cleared: the next solve's barriers would
+// otherwise open before its CTAs have arrived.
+int emit_on_stream(ivp_engine* e, Emitter emit, cudaStream_t s, Prof* prof = nullptr) {
+    Launcher L;
+    L.stream = s;
+    L.prof = prof;
+    L.fail_in = &e->fail_in;
+    const int st = emit(e, L);
+    if (st != IVP_OK && e->persistent) {
+        cudaMemsetAsync(e->D.bar_count, 0, kBarrierWords * sizeof(unsigned), s);
+        cudaGetLastError();
+    }
+    return st;
+}
+
 int run(ivp_engine* e, Emitter emit, cudaGraph_t* g, cudaGraphExec_t* x, cudaStream_t s) {
     if (!e->bound) return IVP_ERR_NOT_BOUND;
     if (e->opt.use_graphs) {
@@ -715,9 +737,7 @@ int run(ivp_engine* e, Emitter emit, cudaGraph_t* g, cudaGraphExec_t* x, cudaStr
         CK(cudaGraphLaunch(*x, s));
         return IVP_OK;
     }
-    Launcher L;
-    L.stream = s;
-    return emit(e, L);
+    return emit_on_stream(e, emit, s);
 }
 
 // Lane count 0: 4 lanes x 64 particles per tile while the dynamic particles
@@ -1408,14 +1428,15 @@ int emit_prj_only(ivp_engine* e, Launcher& L) {
 // A non-pressure force on its own: the kernel of the step where the engine's
 // solves are persistent.  One launch per phase would come back to the host
 // after every CG iteration.
-int force_only(ivp_engine* e, int force, cudaStream_t s) {
-    if (!e->bound) return IVP_ERR_NOT_BOUND;
-    Launcher L;
-    L.stream = s;
+int emit_force_only(ivp_engine* e, Launcher& L, int force) {
     if (!e->persistent) return emit_force(e, L, force);
     CKS(emit_force_persistent(e, L, force));
     return emit_barrier_reset(e, L);
 }
+
+int emit_viscosity_only(ivp_engine* e, Launcher& L) { return emit_force_only(e, L, FORCE_VISC); }
+
+int emit_tension_only(ivp_engine* e, Launcher& L) { return emit_force_only(e, L, FORCE_ST); }
 
 int ivp_ip_solve(ivp_engine* e, void* stream) {
     if (!e) return IVP_ERR_BAD_ARG;
@@ -1429,12 +1450,14 @@ int ivp_prj_solve(ivp_engine* e, void* stream) {
 
 int ivp_viscosity_solve(ivp_engine* e, void* stream) {
     if (!e) return IVP_ERR_BAD_ARG;
-    return force_only(e, FORCE_VISC, as_stream(stream));
+    if (!e->bound) return IVP_ERR_NOT_BOUND;
+    return emit_on_stream(e, emit_viscosity_only, as_stream(stream));
 }
 
 int ivp_surface_tension_solve(ivp_engine* e, void* stream) {
     if (!e) return IVP_ERR_BAD_ARG;
-    return force_only(e, FORCE_ST, as_stream(stream));
+    if (!e->bound) return IVP_ERR_NOT_BOUND;
+    return emit_on_stream(e, emit_tension_only, as_stream(stream));
 }
 
 int ivp_apply_gravity(ivp_engine* e, void* stream) {
@@ -1504,9 +1527,7 @@ int ivp_step_io(ivp_engine* e, const float* x_in, const float* v_in, float* x_ou
         CK(cudaGraphLaunch(e->exec_step_io, s));
         return IVP_OK;
     }
-    Launcher L;
-    L.stream = s;
-    return emit_step_io(e, L);
+    return emit_on_stream(e, emit_step_io, s);
 }
 
 int ivp_read_stats(ivp_engine* e, int32_t scene, void* stream, ivp_solve_stats* out) {
@@ -1584,6 +1605,12 @@ int ivp_set_wait_limit(ivp_engine* e, int64_t ns) {
     return IVP_OK;
 }
 
+int ivp_fail_launch(ivp_engine* e, int32_t n) {
+    if (!e || n < 0) return IVP_ERR_BAD_ARG;
+    e->fail_in = n;
+    return IVP_OK;
+}
+
 int ivp_reset_counters(ivp_engine* e, void* stream) {
     if (!e) return IVP_ERR_BAD_ARG;
     k_reset_counters<<<blocks_for(e->n_scenes, 128), 128, 0, as_stream(stream)>>>(e->D);
@@ -1596,10 +1623,7 @@ int ivp_profile_step(ivp_engine* e, int32_t n_steps, void* stream, double* ms, i
     if (!e->bound) return IVP_ERR_NOT_BOUND;
     cudaStream_t s = as_stream(stream);
     Prof prof;
-    Launcher L;
-    L.stream = s;
-    L.prof = &prof;
-    for (int k = 0; k < n_steps; ++k) CKS(emit_step(e, L));
+    for (int k = 0; k < n_steps; ++k) CKS(emit_on_stream(e, emit_step, s, &prof));
     CK(cudaStreamSynchronize(s));
     for (int k = 0; k < IVP_K_COUNT; ++k) {
         ms[k] = 0.0;

@@ -276,6 +276,11 @@ class Engine:
         (ns <= 0 restores the default of 2 s)."""
         check(self.L.ivp_set_wait_limit(self._handle, int(ns)), "ivp_set_wait_limit")
 
+    def fail_launch(self, n: int):
+        """Test hook: the n-th kernel launched on a stream from now on fails
+        without being launched (0: none)."""
+        check(self.L.ivp_fail_launch(self._handle, int(n)), "ivp_fail_launch")
+
     def reset_counters(self, stream=None):
         check(self.L.ivp_reset_counters(self._handle, ctypes.c_void_p(_stream_ptr(stream))), "ivp_reset_counters")
 

@@ -297,6 +297,11 @@ int ivp_export_neighbours(ivp_engine* e, int32_t scene, int32_t* count, int32_t*
  * only: rebuilds the engine's graphs at their next launch. */
 int ivp_set_wait_limit(ivp_engine* e, int64_t ns);
 
+/* Test hook, no counterpart in the reference.  The n-th kernel that the engine
+ * launches on a stream from now on is not launched, and its call returns
+ * IVP_ERR_CUDA where it stands (0: none).  Launches of graphs do not count. */
+int ivp_fail_launch(ivp_engine* e, int32_t n);
+
 /* Limits of ivp_density_aii_noalloc. */
 #define IVP_NOALLOC_MAX_PARTICLES 65536
 #define IVP_NOALLOC_MAX_CELLS 262144

@@ -2,9 +2,11 @@
 they share holds for the others, in whatever order engines are created and used."""
 import numpy as np
 import pytest
+import torch
 
 import _gpu_helpers as H
 from implicitvelocityprojection_b200 import scenes as S
+from implicitvelocityprojection_b200._lib import IVPError
 
 pytestmark = pytest.mark.gpu
 
@@ -39,3 +41,25 @@ def test_engines_created_later_leave_earlier_ones_working(n, others, use_graphs)
         _solve(e, k)
     for a, b in zip(alone, _solve(eng, n)):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 7])
+@pytest.mark.parametrize("use_graphs", [True, False])
+def test_step_stopped_half_way_leaves_the_engine_usable(use_graphs, n):
+    """A step whose n-th launch fails (before, between and after its solves) leaves
+    their grid barriers ready: the next step is the step of a fresh engine from the
+    state that the failed one left.  A graph's launch cannot stop half-way, so with
+    graphs the failing step is a profiled one."""
+    sc = S.random_column(3000, 2.0, seed=230, viscosity_method=1, viscosity_coeff=1e-3)
+    eng = H.engine([sc], use_graphs=use_graphs, persistent=True)
+    eng.build()
+    eng.fail_launch(n)
+    with pytest.raises(IVPError, match="ivp_fail_launch"):
+        eng.profile_step(1) if use_graphs else eng.step(1)
+    torch.cuda.synchronize()
+    fresh = H.engine([H.with_state(sc, eng.get("x"), eng.get("v"))], use_graphs=use_graphs, persistent=True)
+    for e in (eng, fresh):
+        e.build()
+        e.step(2)
+        assert e.stats(0).status == 0
+    assert np.array_equal(eng.get("x"), fresh.get("x")) and np.array_equal(eng.get("v"), fresh.get("v"))

@@ -714,17 +714,20 @@ int make_graph(ivp_engine* e, Emitter emit, cudaGraph_t* g, cudaGraphExec_t* x) 
     return IVP_OK;
 }
 
-// A call's launches on a stream.  Where they stop half-way, the barrier counters
-// that a solve before left nonzero are cleared: the next solve's barriers would
-// otherwise open before its CTAs have arrived.
+// A call's launches on a stream.  Where they stop half-way, the counters that the
+// kernels behind would have cleared are cleared here: a solve's barriers would
+// otherwise open before its CTAs have arrived, and a build would place particles
+// by the counts of two.
 int emit_on_stream(ivp_engine* e, Emitter emit, cudaStream_t s, Prof* prof = nullptr) {
     Launcher L;
     L.stream = s;
     L.prof = prof;
     L.fail_in = &e->fail_in;
     const int st = emit(e, L);
-    if (st != IVP_OK && e->persistent) {
+    if (st != IVP_OK) {
         cudaMemsetAsync(e->D.bar_count, 0, kBarrierWords * sizeof(unsigned), s);
+        cudaMemsetAsync(e->D.cell_count, 0, sizeof(int) * (size_t)e->n_keys, s);
+        cudaMemsetAsync(e->D.fix_cnt, 0, sizeof(int) * (size_t)e->n_total, s);
         cudaGetLastError();
     }
     return st;

@@ -43,11 +43,11 @@ def test_engines_created_later_leave_earlier_ones_working(n, others, use_graphs)
         assert np.array_equal(a, b)
 
 
-@pytest.mark.parametrize("n", [1, 2, 3, 7])
+@pytest.mark.parametrize("n", [1, 2, 3, 4, 5, 6, 7, 8])
 @pytest.mark.parametrize("use_graphs", [True, False])
 def test_step_stopped_half_way_leaves_the_engine_usable(use_graphs, n):
-    """A step whose n-th launch fails (before, between and after its solves) leaves
-    their grid barriers ready: the next step is the step of a fresh engine from the
+    """A step whose n-th launch fails (before, between and after its solves, and in the build) leaves
+    their grid barriers and the build's counts ready: the next step is the step of a fresh engine from the
     state that the failed one left.  A graph's launch cannot stop half-way, so with
     graphs the failing step is a profiled one."""
     sc = S.random_column(3000, 2.0, seed=230, viscosity_method=1, viscosity_coeff=1e-3)
@@ -63,3 +63,24 @@ def test_step_stopped_half_way_leaves_the_engine_usable(use_graphs, n):
         e.step(2)
         assert e.stats(0).status == 0
     assert np.array_equal(eng.get("x"), fresh.get("x")) and np.array_equal(eng.get("v"), fresh.get("v"))
+
+
+@pytest.mark.parametrize("n", range(1, 13))
+def test_build_stopped_half_way_leaves_the_engine_usable(n):
+    """A build whose n-th launch fails, from the keys to the corrections of lists
+    longer than the cache: the next build and solve are those of a fresh engine."""
+    pts = S.lattice_block([0.1, 0.1, 0.1], (9, 9, 9), 0.0135, jitter=0.1, seed=5)
+    sc = S.assemble([pts], [], particle_radius=0.01, domain_size=[0.5, 0.5, 0.5], max_outer_iters=2,
+                    fixed_outer_iters=True)
+    eng, fresh = (H.engine([sc], use_graphs=False) for _ in range(2))
+    eng.fail_launch(n)
+    with pytest.raises(IVPError, match="ivp_fail_launch"):
+        eng.build()
+    out = []
+    for e in (eng, fresh):
+        e.build()
+        assert e.raw_stats(0).overflow_particles > 0
+        e.solve()
+        out.append([*e.neighbours(0), e.get("density"), e.get("k"), e.get("v")])
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)

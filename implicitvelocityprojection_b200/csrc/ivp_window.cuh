@@ -193,9 +193,10 @@ __device__ __forceinline__ RunOf filter_hits(const WindowGrid& W, BuildShared<SU
 }
 
 // Sums of one particle over its hits.  One reciprocal mass is kept: the
-// dynamic neighbours of a particle nearly always have the same mass.
+// dynamic neighbours of a particle nearly always have the same mass (m_of starts
+// as no mass at all, so that a mass of zero takes its reciprocal too).
 struct HitSums {
-    float rho = 0.0f, aii = 0.0f, m_of = 0.0f, inv_m = 0.0f;
+    float rho = 0.0f, aii = 0.0f, m_of = NAN, inv_m = 0.0f;
     float3 jii = make_float3(0.0f, 0.0f, 0.0f);
 };
 

@@ -8,6 +8,7 @@ import pytest
 
 import _gpu_helpers as H
 from implicitvelocityprojection_b200 import scenes as S
+from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
 
@@ -56,3 +57,24 @@ def test_list_order_sums_are_the_same_bits_at_every_lane_count(scene):
     for lanes, density, k in out[1:]:
         assert np.array_equal(density, out[0][1]), lanes
         assert np.array_equal(k, out[0][2]), lanes
+
+
+@pytest.mark.parametrize("lanes,ppb", LANES)
+@pytest.mark.parametrize("build_kernel", [1, 2])
+def test_neighbour_without_mass_gives_the_reference_k(build_kernel, lanes, ppb):
+    """A dynamic neighbour of mass zero adds 0 / 0 to Aii (pressure_base.py:49-87
+    multiplies |J|^2 by 1 / m): k is NaN around it, as the oracle's, and nowhere
+    else."""
+    sc = _block(1001, 8)
+    sc.density0 = sc.density0.copy()
+    sc.density0[[5, 400]] = 0.0
+    eng = H.engine([sc], lanes_per_particle=lanes, particles_per_block=ppb, build_kernel=build_kernel)
+    eng.build()
+    with np.errstate(divide="ignore", invalid="ignore"):
+        st = O.State.from_scene(sc)
+    st.rebuild()
+    dyn = sc.is_dynamic == 1
+    k, want = eng.get("k")[dyn], st.k[dyn]
+    assert 10 < np.isnan(want).sum() < 200
+    assert np.array_equal(np.isnan(k), np.isnan(want))
+    np.testing.assert_allclose(k[~np.isnan(k)], want[~np.isnan(want)], rtol=1e-5)

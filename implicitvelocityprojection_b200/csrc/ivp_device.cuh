@@ -412,19 +412,12 @@ __device__ __forceinline__ void put_entry(const Dev& D, int row, int k, int j, f
     }
 }
 
-// Fills row entries cnt .. end - 1 with {self, J = 0}, which contribute exactly
-// 0 to every sum: `end` is slice_entries, so that the pair loops need no bounds
-// test.  Lanes `first`, `first + step`, ... of the particle
-// share the entries.
-__device__ __forceinline__ void put_pads(const Dev& D, int row, int cnt, int end, int self, int first, int step) {
-    for (int k = cnt + first; k < end; k += step) put_entry(D, row, k, self, make_float3(0.f, 0.f, 0.f), 0.0f);
-}
-
-// Entries of a row of a slice whose largest row count is cnt_max: whole pairs of
-// every lane.
-__device__ __forceinline__ int slice_entries(const Dev& D, int cnt_max) {
-    const int g = 2 << D.lg;
-    return (cnt_max + g - 1) & ~(g - 1);
+// Fills a row of cnt entries up to whole pairs of every lane with {self, J = 0},
+// which contribute exactly 0 to every sum: the pair loops read that far and need
+// no bounds test.
+__device__ __forceinline__ void put_pads(const Dev& D, int row, int cnt, int self) {
+    const int g = 2 << D.lg, end = (cnt + g - 1) & ~(g - 1);
+    for (int k = cnt; k < end; ++k) put_entry(D, row, k, self, make_float3(0.f, 0.f, 0.f), 0.0f);
 }
 
 // One 32-byte CG record (two float4, 32-byte aligned) in a single 256-bit

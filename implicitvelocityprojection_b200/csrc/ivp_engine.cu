@@ -393,13 +393,12 @@ int emit_build_impl(ivp_engine* e, Launcher& L, bool with_advect) {
             CK(cudaGraphConditionalHandleCreate(&h_fix, L.graph, 0, cudaGraphCondAssignDefault));
             copy.h_fix = (unsigned long long)h_fix;
         }
-        // Build kernel 1 sums density and k in list order: eight slots a warp at
-        // 4 and 8 lanes per particle, 32 at 1 and 2 (many particles: fewer
-        // windows walked).  Build kernel 2 does not; its warps take eight slots
-        // or a slice of rows.  A warp never takes less than a slice, whose rows
-        // it fills up together.
+        // Build kernel 1 sums density and k in list order, build kernel 2 by eight
+        // lanes.  At 1 and 2 lanes per particle, which many particles run, a warp
+        // takes 32 or 16 slots (fewer windows walked: 524,288 particles 339 us by
+        // 16, 379 by eight, 31,007 49 and 38), else eight.
         const bool ordered = e->opt.build_kernel != 2;
-        const int sub = e->G >= 4 ? 8 : ordered || e->G == 1 ? 32 : 16;
+        const int sub = e->G >= 4 ? 8 : ordered ? 32 : 16;
         const void* fn = sub == 32   ? (const void*)k_nbr_build<32, true>
                          : sub == 16 ? (const void*)k_nbr_build<16, false>
                          : ordered   ? (const void*)k_nbr_build<8, true>
@@ -750,9 +749,9 @@ int run(ivp_engine* e, Emitter emit, cudaGraph_t* g, cudaGraphExec_t* x, cudaStr
 constexpr long kAutoTilesPerSM = 16;
 // Build kernel 1 adds density, Aii and J_ii in list order, build kernel 2 by eight
 // lanes; the line keeps each size's sums what one thread per particle and one warp
-// per cell made them.  Kernel 1 costs 3 us more for 768 particles (26 and 23 us),
-// 5 for 31,007 (42 and 38), 18 for 262,144 at 2 lanes per particle (198 and 180)
-// and is 6 faster for 524,288 (333 and 339).
+// per cell made them.  Kernel 1 costs 2 us more for 768 particles (25 and 23 us),
+// 4 for 31,007 (42 and 38), 16 for 262,144 at 2 lanes per particle (196 and 179)
+// and is 6 faster for 524,288 (329 and 335).
 constexpr long kOrderedMinPerSM = 256;
 
 int resolve_options(const ivp_scene_desc* sc, int n, const ivp_options* in, ivp_options* out) {

@@ -462,9 +462,8 @@ __global__ void k_order(const Dev D) {
 // sequential candidate order, so the first cache_size kept are those of the
 // sequential scan.
 //   SUB = 32: each lane walks the bits of its own particle.
-//   SUB = 8, or a slice of rows where that is more: the bits are expanded into
-//   hit lists and eight lanes share a particle; more warps with shorter chains
-//   of loads.
+//   SUB = 8 or 16: the bits are expanded into hit lists and eight lanes share a
+//   particle; more warps with shorter chains of loads.
 // ORDERED adds density, Aii and J_ii in list order, as the reference does (SUB = 32
 // does by its nature): rho - rho0 cancels all but the last digits of the sum, and a
 // constraint near zero falls on one side of the operator's switch or the other.
@@ -716,14 +715,11 @@ __global__ void __launch_bounds__(32 * kBuildWarps) k_nbr_build(const Dev D, int
         }
     }
     __syncwarp();
-    // every row of a slice up to the slice's widest
     const bool act = lane < n;
     const int i = i0 + (act ? lane : 0), row = P.row_base + (i - P.s_begin);
     int pairs = act ? min(found, cap) : 0;
-    int widest = pairs;
-    for (int o = 1; o < (32 >> D.lg); o <<= 1) widest = max(widest, __shfl_xor_sync(0xffffffffu, widest, o));
     if (act) {
-        put_pads(D, row, pairs, slice_entries(D, widest), i, 0, 1);
+        put_pads(D, row, pairs, i);
         const float mi = xl.w;
         float dens = 0.0f;
         dens = dens + mi * P.W0;

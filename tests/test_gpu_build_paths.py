@@ -43,15 +43,17 @@ SCENES = {
 }
 
 
+@pytest.mark.parametrize("build_kernel", [1, 2])
 @pytest.mark.parametrize("scene", sorted(SCENES))
-def test_list_order_sums_are_the_same_bits_at_every_lane_count(scene):
+def test_sums_are_the_same_bits_at_every_lane_count(scene, build_kernel):
     """Build kernel 1 adds density and k in list order: one lane walking its own
     hits (1 and 2 lanes per particle), eight lanes sharing them (4 and 8), and a
-    whole warp on a particle whose window does not fit give the same bits."""
+    whole warp on a particle whose window does not fit give the same bits.  Build
+    kernel 2 adds them by eight lanes, whatever the number of slots a warp takes."""
     sc = SCENES[scene]()
     out = []
     for lanes, ppb in LANES:
-        eng = H.engine([sc], lanes_per_particle=lanes, particles_per_block=ppb, build_kernel=1)
+        eng = H.engine([sc], lanes_per_particle=lanes, particles_per_block=ppb, build_kernel=build_kernel)
         eng.build()
         out.append((lanes, eng.get("density"), eng.get("k")))
     for lanes, density, k in out[1:]:

@@ -1,17 +1,26 @@
 """The neighbour build's branches that ordinary scenes seldom take: windows too
 crowded for the filter pass, particles scattered one per cell (more runs than a
 warp keeps windows for), ragged last tiles and slices, and every number of lanes
-per particle, which sets how many slots a warp takes and how rows interleave.
+per particle, which sets how many slots a warp takes and how rows interleave; the
+solvers over those rows; and the allocation-free density over the same scenes.
+
+Density and k are sums of at most cache_size terms (of one sign, and of J J^T):
+60 additions of 2^-24 each, twice, are 7e-6, and 80 are 1e-5.
 """
+import ctypes
+
 import numpy as np
 import pytest
+import torch
 
 import _gpu_helpers as H
+from implicitvelocityprojection_b200 import _lib
 from implicitvelocityprojection_b200 import scenes as S
 from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
 
+RTOL = 1e-5
 LANES = [(1, 128), (2, 128), (4, 64), (8, 16)]  # lanes per particle, particles per tile
 
 
@@ -43,22 +52,54 @@ SCENES = {
 }
 
 
+def _cells(sc):
+    """Cell of each particle as the build clamps them."""
+    top = np.ceil(np.asarray(sc.domain_size) / sc.support_radius) - 1
+    return np.clip(np.floor(sc.x / sc.support_radius), 0, top).astype(int)
+
+
+def test_scenes_leave_the_filter_pass():
+    """The crowded and the scattered scene are what their names say: 27 cells with
+    more than the filter's 512 candidates, and 32 slots in more than 16 rows of
+    cells."""
+    cells, counts = np.unique(_cells(SCENES["crowded_900"]()), axis=0, return_counts=True)
+    around = (np.abs(cells - cells[counts.argmax()]) <= 1).all(axis=1)
+    assert counts[around].sum() > 512
+    rows = np.sort(_cells(SCENES["scattered_600"]())[:, 1:] @ [1, 1000])
+    assert max(len(np.unique(rows[i:i + 32])) for i in range(0, len(rows) - 32, 32)) > 16
+
+
 @pytest.mark.parametrize("build_kernel", [1, 2])
 @pytest.mark.parametrize("scene", sorted(SCENES))
-def test_sums_are_the_same_bits_at_every_lane_count(scene, build_kernel):
-    """Build kernel 1 adds density and k in list order: one lane walking its own
-    hits (1 and 2 lanes per particle), eight lanes sharing them (4 and 8), and a
-    whole warp on a particle whose window does not fit give the same bits.  Build
-    kernel 2 adds them by eight lanes, whatever the number of slots a warp takes."""
+def test_builds_agree_at_every_lane_count(scene, build_kernel):
+    """The neighbour sets are the oracle's, density and k within rounding of its
+    own.  Over the lane counts the lists are the same entry for entry and the sums
+    the same bits: build kernel 1 adds in list order (one lane walking its own
+    hits at 1 and 2 lanes per particle, eight lanes sharing them at 4 and 8, a
+    whole warp on a particle whose window does not fit), build kernel 2 by eight
+    lanes, whatever the number of slots a warp takes."""
     sc = SCENES[scene]()
-    out = []
+    dyn = np.where(sc.is_dynamic == 1)[0]
+    st = O.State.from_scene(sc)
+    st.rebuild()
+    first = None
     for lanes, ppb in LANES:
-        eng = H.engine([sc], lanes_per_particle=lanes, particles_per_block=ppb, build_kernel=build_kernel)
+        # a list stride that is no whole number of the lanes' pairs
+        eng = H.engine([sc], lanes_per_particle=lanes, particles_per_block=ppb, build_kernel=build_kernel,
+                       list_stride=62)
         eng.build()
-        out.append((lanes, eng.get("density"), eng.get("k")))
-    for lanes, density, k in out[1:]:
-        assert np.array_equal(density, out[0][1]), lanes
-        assert np.array_equal(k, out[0][2]), lanes
+        count, ids = eng.neighbours(0)
+        if first is None:
+            first = (count, ids, eng.get("density"), eng.get("k"))
+            assert H.sets_equal(count, ids, *H.oracle_lists(st), dyn).all()
+            np.testing.assert_allclose(first[2][dyn], st.density[dyn], rtol=RTOL)
+            np.testing.assert_allclose(first[3][dyn], st.k[dyn], rtol=RTOL)
+            other = H.engine([sc], build_kernel=3 - build_kernel)
+            other.build()
+            assert all(np.array_equal(a, b) for a, b in zip(first[:2], other.neighbours(0)))
+            continue
+        for a, b in zip(first, (count, ids, eng.get("density"), eng.get("k"))):
+            assert np.array_equal(a, b), lanes
 
 
 @pytest.mark.parametrize("lanes,ppb", LANES)
@@ -70,13 +111,155 @@ def test_neighbour_without_mass_gives_the_reference_k(build_kernel, lanes, ppb):
     sc = _block(1001, 8)
     sc.density0 = sc.density0.copy()
     sc.density0[[5, 400]] = 0.0
-    eng = H.engine([sc], lanes_per_particle=lanes, particles_per_block=ppb, build_kernel=build_kernel)
-    eng.build()
-    with np.errstate(divide="ignore", invalid="ignore"):
+    with np.errstate(divide="ignore"):
+        eng = H.engine([sc], lanes_per_particle=lanes, particles_per_block=ppb, build_kernel=build_kernel)
         st = O.State.from_scene(sc)
+    eng.build()
     st.rebuild()
     dyn = sc.is_dynamic == 1
     k, want = eng.get("k")[dyn], st.k[dyn]
     assert 10 < np.isnan(want).sum() < 200
     assert np.array_equal(np.isnan(k), np.isnan(want))
-    np.testing.assert_allclose(k[~np.isnan(k)], want[~np.isnan(want)], rtol=1e-5)
+    np.testing.assert_allclose(k[~np.isnan(k)], want[~np.isnan(want)], rtol=RTOL)
+
+
+@pytest.mark.parametrize("row_format", [1, 2])
+@pytest.mark.parametrize("lanes,ppb", LANES + [(8, 32)])
+def test_solves_read_every_interleaving(lanes, ppb, row_format):
+    """Surface tension, viscosity and IP over rows of a ragged scene at every
+    interleaving: persistent and one launch per phase bit for bit, and within the
+    FP32 tolerance of the oracle."""
+    sc = _block(1001, 8)
+    sc.viscosity_method, sc.viscosity_coeff = 1, 1e-3
+    sc.surface_tension_method, sc.surface_tension_coeff = 1, 0.05
+    opts = dict(lanes_per_particle=lanes, particles_per_block=ppb, row_format=row_format, list_stride=62)
+    out = []
+    for persistent in (True, False):
+        eng = H.engine([sc], persistent=persistent, **opts)
+        eng.build()
+        eng.step(1)
+        assert eng.stats(0).status == 0
+        out.append(eng.get("v"))
+    assert np.array_equal(out[0], out[1])
+    assert H.compare_step(sc, **opts)[0]
+
+
+@pytest.mark.parametrize("n_scenes", [1, 2, 3])
+@pytest.mark.parametrize("force", ["viscosity", "tension"])
+def test_force_on_its_own_persistent_equals_per_phase(force, n_scenes):
+    """The implicit forces called on their own, twice, with a step and a solve
+    behind them, in engines of one to three scenes (both kinds of grid barrier):
+    the persistent kernels and one launch per phase give the same bits."""
+    scs = []
+    for i in range(n_scenes):
+        sc = _block(1001 - 300 * i, 9 + i)
+        moving = (sc.is_dynamic == 1)[:, None]
+        sc.v = (np.random.default_rng(i).normal(0.0, 0.1, size=sc.x.shape) * moving).astype(np.float32)
+        if force == "viscosity":
+            sc.viscosity_method, sc.viscosity_coeff = 1, 1e-2
+        else:
+            sc.surface_tension_method, sc.surface_tension_coeff = 1, 0.05
+        scs.append(sc)
+    out = []
+    for persistent in (True, False):
+        eng = H.engine(scs, persistent=persistent)
+        eng.build()
+        for _ in range(2):
+            for _ in range(2):
+                eng.viscosity_solve() if force == "viscosity" else eng.surface_tension_solve()
+            eng.step(1)
+            eng.solve()
+        assert all(eng.stats(i).status == 0 for i in range(n_scenes))
+        out.append([eng.get(q, i) for i in range(n_scenes) for q in ("x", "v")])
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("persistent", [True, False])
+@pytest.mark.parametrize("case", ["not_spd", "not_converged", "no_outer", "prj"])
+def test_divergence_of_a_solve_that_fails(case, persistent):
+    """The divergence output is max(J d / dt, 0) at the last d that the solve
+    reached, whether it ended well or not (and for PRJ's last pass): J d from the
+    lists in 64 bits, d / dt from a solve of the same passes that keeps its v."""
+    from implicitvelocityprojection_b200.engine import Engine, EngineOptions
+    over = {"not_spd": dict(omega=-1.0e4), "not_converged": dict(max_outer_iters=2, density_error_tol=1e-12),
+            "no_outer": dict(max_outer_iters=0, density_error_tol=1e-12),
+            "prj": dict(pressure_method=0, omega=0.5, max_outer_iters=3, fixed_outer_iters=True)}[case]
+    sc = S.column_in_box((8, 10, 8), 0.018, (0.3, 0.4, 0.3), seed=7, **over)
+    moving = (sc.is_dynamic == 1)[:, None]
+    sc.v = (np.random.default_rng(3).normal(0.0, 0.2, size=sc.x.shape) * moving).astype(np.float32)
+
+    def solved(scene):
+        eng = Engine([scene], options=EngineOptions(persistent=persistent), divergence=True)
+        eng.build()
+        eng.prj_solve() if case == "prj" else eng.solve()
+        return eng
+
+    eng = solved(sc)
+    status = eng.raw_stats(0).status
+    assert status == {"not_spd": _lib.NOT_SPD, "prj": 0}.get(case, _lib.NOT_CONVERGED)
+    if case == "not_converged":
+        sc.fixed_outer_iters = True
+        v = solved(sc).get("v").astype(np.float64)
+    else:
+        v = eng.get("v").astype(np.float64)       # (unchanged where the solve fails)
+    count, ids = eng.neighbours(0)
+    h, m, x = float(np.float32(sc.support_radius)), sc.masses()[0].astype(np.float64), sc.x.astype(np.float64)
+    want, size = np.zeros(sc.n), np.zeros(sc.n)
+    for i in np.where(sc.is_dynamic == 1)[0]:
+        j = ids[i, :count[i]]
+        r = x[i] - x[j]
+        d = np.maximum(np.linalg.norm(r, axis=1), 1e-6)
+        J = (-m[j] * 45 / (np.pi * h ** 6) * (h - d) ** 2 / d)[:, None] * r
+        terms = ((v[i] - v[j]) * J).sum(axis=1)
+        want[i] = max(terms.sum(), 0.0)
+        size[i] = ((np.linalg.norm(v[i]) + np.linalg.norm(v[j], axis=1)) * np.linalg.norm(J, axis=1)).sum()
+    assert want.max() > 0
+    # 60 additions and the roundings of J, d and its differences, each 2^-24 of the
+    # terms without cancellation: 5e-6
+    assert (np.abs(eng.get("divergence") - want) <= 5e-6 * size + 1e-12).all()
+
+
+@pytest.mark.parametrize("cache", [60, 80])
+@pytest.mark.parametrize("scene", sorted(SCENES) + ["dense_500"])
+def test_allocation_free_density(scene, cache):
+    """ivp_density_aii_noalloc against direct sums in 64 bits.  dense_500 has more
+    neighbours than a warp's hit lists hold, which only a cache of 80 takes."""
+    if scene == "dense_500":
+        pts = S.lattice_block([0.1, 0.1, 0.1], (8, 8, 8), 0.0165, jitter=0.1, seed=3)[:500]
+        sc = S.assemble([pts], [], particle_radius=0.01, domain_size=[0.5, 0.5, 0.5])
+    else:
+        sc = SCENES[scene]()
+    i = sc.is_dynamic == 1
+    X, M, h = sc.x.astype(np.float64), sc.masses()[0].astype(np.float64), float(np.float32(sc.support_radius))
+    r = X[i][:, None, :] - X[None, :, :]
+    dist = np.sqrt((r ** 2).sum(-1))
+    near = dist < h
+    near[np.arange(int(i.sum())), np.where(i)[0]] = False
+    if scene == "dense_500":
+        assert 64 < near.sum(1).max() <= 80
+        if cache == 60:
+            return  # truncated: which neighbours are kept depends on the candidate order
+    assert near.sum(1).max() <= cache
+    L = _lib.load()
+    dev = torch.device("cuda")
+    x, dyn = torch.from_numpy(sc.x).to(dev), torch.from_numpy(sc.is_dynamic).to(dev)
+    m = torch.from_numpy(sc.masses()[0]).to(dev)
+    density, k = torch.full((sc.n,), -1.0, device=dev), torch.full((sc.n,), -1.0, device=dev)
+    dom = (ctypes.c_float * 3)(*[float(a) for a in sc.domain_size])
+    p = ctypes.c_void_p
+    q = dist / h
+    W = 8 / np.pi / h ** 3 * np.where(q <= 0.5, 6 * (q ** 3 - q ** 2) + 1, 2 * np.clip(1 - q, 0, None) ** 3)
+    rho = M[i] * 8 / np.pi / h ** 3 + (W * near * M).sum(1)
+    rc = np.maximum(dist, 1e-6)
+    J = (-(M * 45 / (np.pi * h ** 6)) * (h - rc) ** 2 / rc * near)[..., None] * r
+    aii = ((J ** 2).sum(-1) * (i / M)).sum(1) + (J.sum(1) ** 2).sum(-1) / M[i]
+    for _ in range(2):
+        assert L.ivp_density_aii_noalloc(p(x.data_ptr()), p(m.data_ptr()), p(dyn.data_ptr()), sc.n,
+                                         ctypes.c_float(sc.particle_radius), ctypes.cast(dom, p), cache,
+                                         p(density.data_ptr()), p(k.data_ptr()),
+                                         p(torch.cuda.current_stream().cuda_stream)) == _lib.OK
+        d, kk = density.cpu().numpy(), k.cpu().numpy()
+        np.testing.assert_allclose(d[i], rho, rtol=RTOL)
+        np.testing.assert_allclose(kk[i], 1 / (aii + 1e-3), rtol=RTOL)
+        assert np.all(kk[~i] == 0.0) and np.all(d[~i] == -1.0)

@@ -577,7 +577,7 @@ def run_ours(args, rank, world, local_rank):
                            "particles_per_block": ppb,
                            "solve": "persistent cooperative kernel" if opts.persistent else "per-phase launches",
                            "launch_shape": "autotuned" if tuning else ("fixed" if args.lanes else "heuristic"),
-                           "build_kernel": {1: "thread per particle", 2: "warp per cell"}[build_kernel],
+                           "build_kernel": {1: "sums in list order", 2: "sums by eight lanes"}[build_kernel],
                            "timed": schedule_note(args.warmup, args.steps, run_steps)},
                 "p50_ms": float(np.percentile(step_ms, 50)), "p99_ms": float(np.percentile(step_ms, 99)),
                 "valid": bool(valid), "max_final_density_error": max(r.max_final_density_error for r in raws),
@@ -860,7 +860,7 @@ def main():
     ap.add_argument("--row-format", default="full", choices=sorted(ROW_FORMATS),
                     help="neighbour rows: full FP32 gradients (default), compact {j, w}, or bf16 gradients")
     ap.add_argument("--build-kernel", type=int, default=0, choices=[0, 1, 2],
-                    help="neighbour build: 0 chosen from the scenes, 1 one thread per particle, 2 one warp per cell")
+                    help="neighbour build: 0 chosen from the scenes, density and k summed 1 in list order, 2 by eight lanes")
     ap.add_argument("--no-autotune", action="store_true",
                     help="skip the launch-shape autotuner (use the engine's tile-count heuristic)")
     ap.add_argument("--shard", action="store_true",

@@ -35,8 +35,11 @@ SHAPES: Tuple[Tuple[int, int], ...] = ((2, 128), (4, 64), (8, 32), (2, 64), (4, 
 # compact {j, w_ij} (8 B, J rebuilt from the positions).  Full rows win while
 # the rows stay in L2; compact rows halve the row stream once they do not.
 ROW_FORMATS: Tuple[int, ...] = (1, 2)
-# neighbour builds with identical lists: density in list order, by eight lanes
+# neighbour builds with identical lists: density and k in list order, by eight
+# lanes.  Stored results and their readers know them by the names of the first
+# two kernels that were timed against each other here.
 BUILD_KERNELS: Tuple[int, ...] = (1, 2)
+BUILD_NAMES = {1: "thread per particle", 2: "warp per cell"}
 BUILD_REPS = 5
 
 _CACHE: Dict[str, dict] = {}
@@ -162,7 +165,7 @@ def tune(scenes: Sequence, device: str = "cuda", base_options=None, warmup: int 
                       "build_kernel": min(build_ms, key=build_ms.get) if build_ms else base.build_kernel},
            "table": [{"shape": tr.label(), "ms_per_step": tr.ms_per_step} for tr in trials],
            "build_ms": None if build_ms is None else
-           {{1: "thread per particle", 2: "warp per cell"}[bk]: ms for bk, ms in build_ms.items()},
+           {BUILD_NAMES[bk]: ms for bk, ms in build_ms.items()},
            "tuning_s": round(time.perf_counter() - t0, 2), "steps_timed": steps}
     _CACHE[key] = res
     if cache_file:

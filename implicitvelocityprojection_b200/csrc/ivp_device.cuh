@@ -256,8 +256,6 @@ struct Dev {
     // the viscosity kernel applies the step's gravity in its prologue (set on
     // step launches whose first force is the viscosity; k_gravity is then skipped)
     int fold_gravity;
-    // the persistent solve runs the viscosity phases (set on step launches)
-    int visc_enabled;
     int force;               // implicit non-pressure solve of this launch: 0 viscosity, 1 surface tension
     int bar_all_reduce;      // persistent solve: every CTA reduces the (few) partials itself
     // persistent solve: grid-barrier words and the phase budget.  Every kind of
@@ -291,14 +289,6 @@ __device__ __forceinline__ float cubic_W(float r, float h, float k) {
         }
     }
     return res;
-}
-
-// sph_kernel.py:52-61 as a weight: grad W(r) = w * r with
-// w = -k (h - |r|)^2 / max(|r|, 1e-6)
-__device__ __forceinline__ float spiky_w(float rn, float h, float k) {
-    float rc = rn < 1e-6f ? 1e-6f : rn;
-    float t = h - rc;
-    return (-k * (t * t)) / rc;
 }
 
 // |r|^2 rounded exactly as the reference's wp.length computes it before the
@@ -347,7 +337,11 @@ __device__ __forceinline__ float group_sum(float v) {
 
 constexpr int ROW_FULL = 0, ROW_COMPACT = 1, ROW_BF16 = 2;
 // How a kernel reads the rows: full rows that stay in L2, full rows that
-// stream from DRAM (Dev::row_stream), or whatever Dev::row_fmt says.
+// stream from DRAM (Dev::row_stream), or whatever Dev::row_fmt says.  The
+// persistent solves are compiled for one of the three.  IP solve by READ_FULL and
+// by READ_ANY: 102,400 particles 347 and 359 us, 31,007 195 and 201; by
+// READ_STREAM, READ_ANY and READ_FULL: 262,144 929, 943 and 1,068 us, 524,288
+// 1,310, 1,328 and 1,406.
 constexpr int READ_FULL = 0, READ_STREAM = 1, READ_ANY = 2;
 
 

@@ -403,11 +403,9 @@ int emit_build_impl(ivp_engine* e, Launcher& L, bool with_advect) {
                          : sub == 16 ? (const void*)k_nbr_build<16, false>
                          : ordered   ? (const void*)k_nbr_build<8, true>
                                      : (const void*)k_nbr_build<8, false>;
-        const int warps = e->n_tiles * blocks_for(e->T, sub);
         int T = e->T;
         void* args[] = {&copy, &T};
-        CKS(L.kernel(IVP_K_NBR_BUILD, fn,
-                     dim3(blocks_for(warps, kBuildWarps)), dim3(32 * kBuildWarps), args));
+        CKS(L.kernel(IVP_K_NBR_BUILD, fn, dim3(e->n_tiles * blocks_for(e->T, sub)), dim3(32), args));
         if (L.graph) {
             cudaGraph_t body;
             CKS(add_conditional(L.graph, L, h_fix, cudaGraphCondTypeIf, &body));
@@ -583,14 +581,13 @@ int emit_force(ivp_engine* e, Launcher& L, int force) {
     return L.dev(kid, K.v_end, nt, B, D0);
 }
 
-int emit_solve(ivp_engine* e, Launcher& L, bool with_visc = false) {
+int emit_solve(ivp_engine* e, Launcher& L) {
     if (e->n_tiles == 0 || !e->any_ip) return IVP_OK;
     if (e->persistent) {
         KernelSet K;
         kernel_set(e->G, e->BLOCK, row_read(e->D), e->n_scenes, &K);
         Dev copy = e->D;
         copy.bar_count += BAR_IP;
-        copy.visc_enabled = with_visc ? 1 : 0;
         void* args[] = {&copy};
         return L.kernel(IVP_K_PERSISTENT, (const void*)K.persist, dim3(e->coop_grid), dim3(e->BLOCK), args,
                         e->coop_smem, true);
@@ -648,7 +645,7 @@ int emit_step(ivp_engine* e, Launcher& L) {
         CKS(L.dev(IVP_K_GRAVITY, k_gravity, blocks_for(e->n_total, ELEM_BLOCK), ELEM_BLOCK, e->D));
         CKS(emit_forces(e, L));
     }
-    CKS(emit_solve(e, L, true));
+    CKS(emit_solve(e, L));
     CKS(emit_prj(e, L));
     CKS(emit_build_impl(e, L, true));  // advection (skipping scenes whose solve failed) + the next build
     return IVP_OK;
@@ -745,7 +742,10 @@ int run(ivp_engine* e, Emitter emit, cudaGraph_t* g, cudaGraphExec_t* x, cudaStr
 // Lane count 0: 4 lanes x 64 particles per tile while the dynamic particles
 // fill at most kAutoTilesPerSM tiles of 64 per SM, else 2 lanes x 128.  With
 // many tiles per CTA the persistent solves walk fewer, larger tiles per phase
-// (one block reduction per tile); with few, 4 lanes split each row wider.
+// (one block reduction per tile); with few, 4 lanes split each row wider.  IP
+// solve at 4 x 64 and at 2 x 128: 768 particles 90 and 103 us, 8,192 106 and 117,
+// 31,007 197 and 191, 102,400 359 and 347, 262,144 1,018 and 945, 524,288 1,567
+// and 1,314; the build at 4 x 64 is faster up to 102,400 (105 and 115 us).
 constexpr long kAutoTilesPerSM = 16;
 // Build kernel 1 adds density, Aii and J_ii in list order, build kernel 2 by eight
 // lanes; the line keeps each size's sums what one thread per particle and one warp
@@ -1418,7 +1418,7 @@ int emit_barrier_reset(ivp_engine* e, Launcher& L) {
 }
 
 int emit_ip_only(ivp_engine* e, Launcher& L) {
-    CKS(emit_solve(e, L, false));
+    CKS(emit_solve(e, L));
     return emit_barrier_reset(e, L);
 }
 

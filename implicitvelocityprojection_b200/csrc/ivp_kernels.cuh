@@ -448,7 +448,9 @@ __global__ void k_order(const Dev D) {
 // diagonal k = 1/(Aii + 1e-3) (pressure_base.py:49-87) and the constraint
 // c = rho - rho0 (pressure_base.py:169-184).
 //
-// One warp takes SUB consecutive dynamic slots and works in two passes.
+// One warp takes SUB consecutive dynamic slots and works in two passes.  It is a
+// CTA of its own: warps share nothing, and a CTA's slot on its SM is free as soon
+// as its warp is done (524,288 particles: 332 us, two warps per CTA 351, four 372).
 //
 // Filter: the slots are sorted by cell, so the warp's particles are a few runs
 // of one cell each (or of a few thinly filled x-adjacent cells), and the
@@ -470,7 +472,6 @@ __global__ void k_order(const Dev D) {
 // Lanes that share a particle then pass their hits' factors through shared memory
 // to one chain per sum (ListOrder).  At 4 lanes per particle: 98 us for 102,400
 // particles (87 by eight lanes), 69 (62) for 60,000, 26 (23) for 768.
-constexpr int kBuildWarps = 1;  // warps per CTA: they share nothing, and a CTA's slot is free as soon as its warp is done
 
 // N lanes (8 or 32) sum the n_hit hits of a particle in list order: `take(k, a, W,
 // jj, J)` computes hit k and returns m_j.  n_hit is the same in the N lanes; the
@@ -518,14 +519,15 @@ __device__ __forceinline__ int scan_alone(const WindowGrid& W, int* list, int i,
 }
 
 template <int SUB, bool ORDERED>
-__global__ void __launch_bounds__(32 * kBuildWarps) k_nbr_build(const Dev D, int tile_size) {
-    __shared__ BuildShared<SUB> sh[kBuildWarps];
-    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    BuildShared<SUB>& S = sh[wid];
+__global__ void __launch_bounds__(32) k_nbr_build(const Dev D, int tile_size) {
+    __shared__ BuildShared<SUB> S;
+    // (the mask and the guard below change nothing but the registers, 66 to 72;
+    // without them ptxas stops at 64, and 262,144 particles take 208 us, not 196)
+    const int lane = threadIdx.x & 31;
     const int per_tile = (tile_size + SUB - 1) / SUB;
-    const int gw = blockIdx.x * kBuildWarps + wid;
+    const int gw = blockIdx.x;
     const int t = gw / per_tile;
-    if (t >= D.n_tiles) return;  // warp-uniform; the kernel has no CTA barrier
+    if (t >= D.n_tiles) return;
     const int4 tile = __ldg(D.tiles + t);
     const int i0 = tile.y + (gw - t * per_tile) * SUB;
     const int n = min(SUB, tile.z - i0);
@@ -1910,7 +1912,6 @@ __device__ __forceinline__ double st_a_tile(const Dev& D, const SceneParams& P, 
         zi = f3(D.stz[T.i]);
     }
     float sx = 0.f, sy = 0.f, sz = 0.f;
-    const int self = T.valid ? T.i : P.s_begin;
     // the entries where `each` reads the rows', {j, w} of a pair in 16 bytes
     const int lane = threadIdx.x & 31;
     const float4* q = reinterpret_cast<const float4*>(D.st_w + (size_t)(T.row - lane / G) * D.stride) + lane;
@@ -2922,10 +2923,9 @@ __global__ void k_reset_counters(const Dev D) {
     if (s == 0) D.flags->timeout = 0;
 }
 
-// Neighbour lists of one scene in the reference layout, original indices.
-// One scene's statistics and histories gathered into the staging block
-// (StatStage), so the host reads them with one copy.  One CTA, 4-byte words
-// (every part is a multiple of 4 bytes).
+// One scene's statistics and histories, written into the staging block
+// (StatStage) in page-locked host memory.  One CTA, 4-byte words (every part is a
+// multiple of 4 bytes).
 __device__ __forceinline__ void copy_words(unsigned char* dst, const void* src, size_t bytes) {
     const unsigned* s = static_cast<const unsigned*>(src);
     unsigned* d = reinterpret_cast<unsigned*>(dst);
@@ -2943,6 +2943,7 @@ __global__ void k_stage_stats(const Dev D, int scene, int hist) {
     copy_words(D.stage + L.pcg, D.pcg_hist + (size_t)scene * hist, sizeof(int) * (size_t)hist);
 }
 
+// Neighbour lists of one scene in the reference layout, original indices.
 __global__ void k_export(const Dev D, int scene, int* count, int* ids, int cache) {
     const SceneParams& P = D.scenes[scene];
     const int i = P.s_begin + blockIdx.x * blockDim.x + threadIdx.x;

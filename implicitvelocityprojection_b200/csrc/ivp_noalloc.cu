@@ -113,17 +113,15 @@ __global__ void na_order(const float* __restrict__ x, const float* __restrict__ 
 //
 // One warp per eight slots, as in the engine's build for small scenes: a thread
 // per particle walked 270 candidates one after another, on 176 CTAs of 256
-// threads for 40,000 particles (99 us), and left most of the chip waiting.  One warp per CTA: 60 us a call;
-// two: 63 to 73.
-constexpr int kSub = 8, kWarps = 1;
+// threads for 40,000 particles (99 us), and left most of the chip waiting.  One
+// warp per CTA: 60 us a call; two: 63 to 73.
+constexpr int kSub = 8;
 
-__global__ void __launch_bounds__(32 * kWarps) na_density_aii(int n, Grid g, Scratch* S, float* __restrict__ density,
-                                                              float* __restrict__ kdiag) {
-    __shared__ ivp::BuildShared<kSub> sh[kWarps];
-    const int lane = threadIdx.x & 31;
-    ivp::BuildShared<kSub>& B = sh[threadIdx.x >> 5];
-    const int i0 = (blockIdx.x * kWarps + (threadIdx.x >> 5)) * kSub;
-    if (i0 >= n) return;  // warp-uniform; the kernel has no CTA barrier
+__global__ void __launch_bounds__(32) na_density_aii(int n, Grid g, Scratch* S, float* __restrict__ density,
+                                                     float* __restrict__ kdiag) {
+    __shared__ ivp::BuildShared<kSub> B;
+    const int lane = threadIdx.x;
+    const int i0 = blockIdx.x * kSub;
     const int n_dyn = S->cell_start[g.ncell];
     if (lane < kSub && i0 + lane < n && i0 + lane >= n_dyn) kdiag[S->pid[i0 + lane]] = 0.0f;
     const int m = min(kSub, n_dyn - i0);
@@ -305,8 +303,7 @@ extern "C" int ivp_density_aii_noalloc(const float* x, const float* m, const int
     if (st == IVP_OK) st = launch((const void*)ivp::k_scan_add, nsb, ivp::SCAN_BLOCK, a_scan2, s, "scan_add");
     if (st == IVP_OK) st = launch((const void*)na_place, nb, B, a_place, s, "na_place");
     if (st == IVP_OK) st = launch((const void*)na_order, nb, B, a_order, s, "na_order");
-    if (st == IVP_OK) st = launch((const void*)na_density_aii, (n + kSub * kWarps - 1) / (kSub * kWarps), 32 * kWarps, a_dens, s,
-                                   "na_density_aii");
+    if (st == IVP_OK) st = launch((const void*)na_density_aii, (n + kSub - 1) / kSub, 32, a_dens, s, "na_density_aii");
     if (st != IVP_OK) return st;
     return IVP_OK;
 }

@@ -32,7 +32,7 @@ class EngineOptions:
     use_graphs: bool = True
     persistent: bool = True
     row_format: int = 0  # 0 default (full), 1 full {J, j}, 2 compact {j, w}, 3 bf16 gradients
-    build_kernel: int = 0  # density summed 1 in list order, 2 by eight lanes; 0: chosen from the scenes
+    build_kernel: int = 0  # density and k summed 1 in list order, 2 by eight lanes; 0: chosen from the scenes
 
     def to_c(self) -> _lib.Options:
         o = _lib.Options()

@@ -38,7 +38,7 @@ typedef enum {
     IVP_ERR_CUDA = 5,
     IVP_ERR_TIMEOUT = 6,
     IVP_ERR_NOT_BOUND = 7,      /* particle arrays not bound */
-    IVP_ERR_DEVICE_CHECK = 8    /* a device-side bounds check failed (index out of range) */
+    IVP_ERR_DEVICE_CHECK = 8    /* the build found a particle's slot outside its scene, or is_dynamic at odds with n_dynamic */
 } ivp_status;
 
 /* One independent scene.  Its particles occupy [particle_offset,
@@ -83,9 +83,8 @@ typedef struct {
                                      positions: half the list memory, slower; bit-identical to 1),
                                      3 bf16 (4 B id + the gradient in 3 bf16: the reduced-precision
                                      variant, 10 B per entry) */
-    int32_t build_kernel;         /* neighbour build: 1 density summed in list order (32 particles per
-                                     warp at 1 and 2 lanes per particle), 2 summed by eight lanes;
-                                     the same lists in the same order.  0 (default): chosen from the
+    int32_t build_kernel;         /* neighbour build: 1 density and k summed in list order, 2 summed by
+                                     eight lanes; the same lists in the same order.  0 (default): chosen from the
                                      scenes (1 from 256 dynamic particles per SM) */
 } ivp_options;
 
@@ -314,8 +313,8 @@ int ivp_fail_launch(ivp_engine* e, int32_t n);
  * cudaMalloc/cudaFree.  It allocates nothing and
  * needs no workspace: its scratch is one fixed device array inside the
  * library (about 6.3 MB, held on every GPU that loads the library until the
- * process exits).  Results equal those of ivp_neighbour_build for the same
- * particles.  Inputs: x float[n][3], m float[n], is_dynamic int[n] (caller
+ * process exits).  Results are those of ivp_neighbour_build for the same
+ * particles up to the order of their sums.  Inputs: x float[n][3], m float[n], is_dynamic int[n] (caller
  * order, device pointers); outputs density[n], kdiag[n] (density of static
  * particles is left untouched).  At most IVP_NOALLOC_MAX_PARTICLES particles
  * and IVP_NOALLOC_MAX_CELLS cells of size h = 4 r over the domain; larger

@@ -721,9 +721,9 @@ def test_autotuner_picks_a_candidate_and_caches():
 
 @pytest.mark.parametrize("scene", ["column", "dam", "overflow"])
 def test_build_kernels_same_lists(golden_dir, scene):
-    """The thread-per-particle build and the warp-per-cell build walk the
-    candidates in the same order: identical neighbour lists entry for entry
-    (also with truncated lists), density and k equal up to their summation
+    """The build that sums in list order and the build that sums by eight lanes
+    walk the candidates in the same order: identical neighbour lists entry for
+    entry (also with truncated lists), density and k equal up to their summation
     order, and steps equal within the FP32 tolerance."""
     if scene == "column":
         sc = S.column_in_box((12, 24, 12), 0.02, (0.4, 1.0, 0.4), seed=4, viscosity_method=1, viscosity_coeff=1e-3)

@@ -199,7 +199,9 @@ int ivp_ip_solve(ivp_engine* e, void* stream);
 /* Weiler18.solve(coeff, dt) (scripts/sim/forces/non_pressure/viscosity/
  * weiler18.py:371-401): implicit viscosity with block-Jacobi PCG for every
  * scene whose viscosity_method is 1 and viscosity_coeff > 0; updates the bound
- * velocities.  Uses the current neighbour lists and densities. */
+ * velocities.  Uses the current neighbour lists and densities.  Asynchronous
+ * where the engine's solves are persistent; one launch per phase returns to the
+ * host after every CG iteration. */
 int ivp_viscosity_solve(ivp_engine* e, void* stream);
 
 /* Jeske23.solve(sigma, sigma, dt) (scripts/sim/forces/non_pressure/
@@ -207,7 +209,7 @@ int ivp_viscosity_solve(ivp_engine* e, void* stream);
  * PCG for every scene whose surface_tension_method is 1 and
  * surface_tension_coeff > 0; updates the bound velocities.  Uses the current
  * neighbour lists and densities.  ivp_step runs it after gravity and before
- * the viscosity (framework.py:400-421). */
+ * the viscosity (framework.py:400-421).  Asynchronous as ivp_viscosity_solve. */
 int ivp_surface_tension_solve(ivp_engine* e, void* stream);
 
 /* PRJ.solve(dt) (scripts/sim/forces/pressure/prj.py:296-340): projected
